@@ -194,20 +194,25 @@ SNN_API int snn_get_timing(snn_handle *h, double *score_ms, int *score_launches,
                            int *commit_launches, double *total_ms, int *total_launches);
 
 /* Options:
- *   SNN_OPT_KERNEL scoring kernel: 0 automatic (3 for k_max <= 64, else 1),
- *                  1 rows per lane (any k_max <= 256), 3 row tiles fed by a
- *                  TMA/mbarrier ring (k_max <= 64).  Results are identical;
- *                  this exists for cross-checks and measurement. */
+ *   SNN_OPT_KERNEL scoring kernel: 0 automatic (a pruned scan for steps that
+ *                  have starting bounds -- forward steps from seed columns,
+ *                  backward steps after the first -- else 3 for k_max <= 64,
+ *                  else 1), 1 rows per lane (any k_max <= 256), 3 row tiles
+ *                  fed by a TMA/mbarrier ring (k_max <= 64).  Results are
+ *                  identical; this exists for cross-checks and measurement. */
 #define SNN_OPT_KERNEL 2
 /*   SNN_OPT_COUNTERS 1: the TMA-fed scorer keeps the filter counters read by
- *                  snn_get_filter_counters (a little slower).  Default 0. */
+ *                  snn_get_filter_counters; it then scores the steps that the
+ *                  automatic choice would give to the pruned scan.  Default 0. */
 #define SNN_OPT_COUNTERS 3
 /*   SNN_OPT_SEED_STEP forward step (= features already committed) from which
- *                  the TMA-fed scorer takes each candidate's starting bound on
- *                  its k-th neighbour distance from 256 "seed" columns near
- *                  the row (kept by the previous commit) instead of a first
- *                  pass over a quarter of the columns.  Results are identical;
- *                  only the work differs.  Default 2 (3 when k_max > 16); a
+ *                  each candidate's starting bound on its k-th neighbour
+ *                  distance comes from 256 "seed" columns near the row (kept
+ *                  by the previous commit) instead of a first pass over a
+ *                  quarter of the columns; steps with such bounds are scored
+ *                  by the pruned scan.  Results are identical; only the work
+ *                  differs.  Default 2 for a holdout problem with k_max <= 64
+ *                  (its first two steps run from sorted columns), else 1; a
  *                  large value turns it off. */
 #define SNN_OPT_SEED_STEP 4
 /*   SNN_OPT_SORTED_START 1 (default): the first two forward steps of a

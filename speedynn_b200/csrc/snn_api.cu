@@ -104,6 +104,9 @@ struct snn_handle {
     char *stemp = nullptr;
     size_t stemp_bytes = 0;
     unsigned long long *walked = nullptr;  // columns walked by the sorted second step
+    float *xg = nullptr;          // pruned scan: packed candidates [ceil(p / 32)][ldc][32]
+    float2 *ext = nullptr;        // backward: [ceil(p / 32)][ldc] column extremes
+    float4 *fstat = nullptr;      // backward: per-feature mean and range
     bool sorted_start = true;     // SNN_OPT_SORTED_START
     bool seeds_ok = false;        // seeds hold the current D's seed columns
     int seed_step = 2;            // SNN_OPT_SEED_STEP: first forward step scored from seed bounds (set at create)
@@ -171,6 +174,9 @@ struct snn_handle {
         b.seed_d = seed_d;
         b.bound = sbound;
         b.use_seeds = 0;
+        b.xg = xg;
+        b.ext = ext;
+        b.fstat = fstat;
         b.only_if_full = 0;
         return b;
     }
@@ -228,7 +234,7 @@ void free_all(snn_handle *h)
                         h->err, h->stage, h->rmse64, h->err64, h->kv, h->cands, h->prev_cands, h->mask, h->order,
                         h->stepk, h->st, h->nn_idx, h->nn_dist, h->seeds, h->seed_d, h->sbound, h->sval, h->skey, h->sidx,
                         h->sord, h->soff, h->stemp, h->walked, h->perm, h->fvar,
-                        h->d_loss_ids, h->lossval, h->err_all, h->kth_prev, h->dmax, h->fcount};
+                        h->d_loss_ids, h->lossval, h->err_all, h->kth_prev, h->dmax, h->fcount, h->xg, h->ext, h->fstat};
         for (void *q : ptrs)
             if (q) cudaFree(q);
     }
@@ -275,18 +281,25 @@ int check_device(int device)
 bool use_tma(const snn_handle *h) { return h->kernel == 3 || (h->kernel == 0 && snn::score_tma_supported(h->kmax)); }
 
 // Forward step t (t features committed) is scored from seed bounds once
-// t >= seed_step: after two commits the columns nearest under D are mostly
-// near under D + one more feature too, and the bound over 256 of them beats a
-// first pass over a quarter of the columns (on the fwd-64k data, rows whose
-// filter fires: 17.9 % against 21.5 % at step 2, 6.9 % against 12.1 % at
-// step 14; at step 1, with one feature committed, the first pass is better).
-// With k above 16 the seeds start a step later: a k-th distance over the
-// seeds needs them to be near in more features (fwd-200k, k = 50: step 2
-// took 913 ms seeded against 845 ms with the first pass, step 3 767 against
-// 825).  The commit before such a step writes the seeds.
+// t >= seed_step: the columns nearest under D are mostly near under D + one
+// more feature too, so any k of 256 of them bound the k-th distance well.  The
+// sorted columns of a holdout problem score its first two steps (k <= 64)
+// faster; everything else starts with the first step that has a commit behind
+// it (step 1 of a 3000-row CV problem: 0.23 ms by the scan from seed bounds,
+// 0.57 ms dense with a first pass; step 2 of fwd-64k: 9.9 against 31 ms).  The
+// commit before such a step writes the seeds.
 bool seeds_for_step(const snn_handle *h, int t)
 {
-    return !h->desc.backward && h->seeds && use_tma(h) && t >= h->seed_step;
+    return !h->desc.backward && h->seeds && h->kernel != 1 && t >= h->seed_step;
+}
+
+// The automatic choice scores a step by the pruned scan (snn_scan.cu) once it
+// has starting bounds: forward from seed columns, backward from the previous
+// step's k-th distances.  The filter counters and the injected stall belong to
+// the TMA-fed scorer, so a step that wants them takes that one.
+bool scan_step(const snn_handle *h)
+{
+    return h->kernel == 0 && snn::scan_supported(h->n_cols, h->kmax) && !(h->count_filter || h->inject_stall >= 0) && (h->desc.backward ? h->prev_ok : h->seeds_ok);
 }
 
 // The first two forward steps of a holdout problem run from sorted feature
@@ -316,29 +329,33 @@ int issue_step(snn_handle *h, int t)
         h->inject_launch = -1;
         return fail(SNN_ERR_CUDA, "injected launch failure at step %d", t);
     }
-    bool tma_step = false;
     if (sorted_step(h, t)) {
         if (t == 0) SNN_CUDA(snn::launch_first_step(b, h->sval, h->sidx, n_cand, h->stream));
         else SNN_CUDA(snn::launch_second_step(b, h->sval, h->sidx, h->skey, n_cand, h->walked, h->stream));
         b.only_if_full = 1;  // the scan below runs only if some tie group was too large
         h->n_launch += t == 0 ? 1 : 2;  // the second step gathers the candidates in sorted order first
     }
-    if (use_tma(h)) {
+    const bool seeded = !backward && h->seeds_ok && seeds_for_step(h, t);
+    bool prev = false;  // this step writes every candidate's k-th distances (backward)
+    const bool scan = !b.only_if_full && scan_step(h) && (backward || seeded);
+    if (scan || (seeded && use_tma(h))) {
+        SNN_CUDA(snn::launch_pack_groups(b, n_cand, backward, h->stream));
+        if (seeded) SNN_CUDA(snn::launch_seed_bounds(b, n_cand, h->stream));
+        h->n_launch += seeded ? 2 : 1;
+    }
+    if (scan) {
+        SNN_CUDA(snn::launch_scan(b, n_cand, backward, h->max_smem, h->stream));
+        prev = backward;
+    } else if (use_tma(h)) {
         b.use_prev = backward && h->prev_ok ? 1 : 0;
-        b.use_seeds = seeds_for_step(h, t) && h->seeds_ok ? 1 : 0;
+        b.use_seeds = seeded ? 1 : 0;
         if (!b.only_if_full) {  // the injected stall goes to a launch that scans
             b.inject_stall = h->inject_stall + 1;  // 0: off
             h->inject_stall = -1;
         }
-        if (b.use_seeds) {
-            // the sort's value buffer (p x ldc, unused after load) holds the row-major candidates
-            SNN_CUDA(snn::launch_seed_bounds(b, n_cand, reinterpret_cast<float *>(h->sord), h->stream));
-            h->n_launch += h->kmax <= 16 && h->sord ? 2 : 1;
-        }
         SNN_CUDA(snn::launch_score_tma(b, n_cand, backward, h->stream));
         h->n_launch += snn::score_tma_launches(h->kmax, n_cand, backward) - 1;  // counted once below
-        h->prev_ok = backward && h->kth_prev;  // this step wrote every candidate's k-th distances
-        tma_step = true;
+        prev = backward && h->kth_prev;
     } else {
         SNN_CUDA(snn::launch_score(b, n_cand, h->plan, backward, h->stream));
     }
@@ -346,7 +363,7 @@ int issue_step(snn_handle *h, int t)
         SNN_CUDA(cudaEventRecord(se->b, h->stream));
         h->n_score++;
     }
-    if (!tma_step) h->prev_ok = false;
+    h->prev_ok = prev;
     if (h->model == 1) {
         SNN_CUDA(snn::launch_mode_predict(b, n_cand, h->stream));
         h->n_launch += 1;
@@ -466,6 +483,8 @@ static size_t handle_bytes(const snn_desc *d, int kmax)
     // sorted feature columns of the first forward step and the sort's buffers
     if (!d->backward && !cv) f += 4 * p * ldc + 2 * p + snn::sort_temp_bytes(d->p, (int)ldc) / sizeof(float) + 1;
     if (d->backward) f += p * n_rows + n_rows;  // kth_prev, dmax
+    const size_t groups = (p + 31) / 32;         // packed candidates of the pruned scan, backward: their extremes
+    f += groups * ldc * 32 + (d->backward ? 2 * groups * ldc + 4 * p : 0);
     if (!cv) f += p * ldr;
     return sizeof(float) * f + ((size_t)1 << 20);
 }
@@ -497,7 +516,7 @@ SNN_API int snn_create(const snn_desc *d, snn_handle **out)
     h->n_rows = cv ? d->n_train : d->n_val;
     h->npf = cv ? d->n_train / d->k_fold : 1;
     h->kmax = kmax;
-    h->seed_step = kmax <= 16 ? 2 : 3;
+    h->seed_step = cv || kmax > 64 ? 1 : 2;
     h->nk = d->num_k_vals;
     h->ldc = round_up(h->n_cols, snn::kPadCols);
     h->ldr = cv ? h->ldc : round_up(h->n_rows, snn::kPadCols);
@@ -556,6 +575,10 @@ SNN_API int snn_create(const snn_desc *d, snn_handle **out)
         if ((rc = dev_alloc(&h->seed_d, (size_t)h->n_rows * snn::kSeeds, "seed distances"))) return bail(rc);
         if ((rc = dev_alloc(&h->sbound, p * h->n_rows, "seed bounds"))) return bail(rc);
     }
+    const size_t groups = (p + 31) / 32;
+    if ((rc = dev_alloc(&h->xg, groups * h->ldc * 32, "packed candidates"))) return bail(rc);
+    if (d->backward && (rc = dev_alloc(&h->ext, groups * h->ldc, "column extremes"))) return bail(rc);
+    if (d->backward && (rc = dev_alloc(&h->fstat, p, "feature ranges"))) return bail(rc);
     if (!d->backward && !cv) {
         const size_t pl = p * h->ldc;
         if ((rc = dev_alloc(&h->sval, pl, "sorted values"))) return bail(rc);
@@ -615,7 +638,7 @@ static int load_impl(snn_handle *h, const float *X_train, const float *y_train, 
     // candidate slot order: ascending training variance, so that the four
     // candidates a scoring warp shares a filter bound with have distances of
     // similar scale (any order gives the same results)
-    SNN_CUDA(snn::launch_feature_variance(h->bufs(), h->fvar, h->stream));
+    SNN_CUDA(snn::launch_feature_variance(h->bufs(), h->fvar, h->fstat, h->stream));
     SNN_CUDA(snn::launch_feature_order(h->fvar, h->p, h->perm, h->stream));
     if (h->sval)
         SNN_CUDA(snn::launch_sort_features(h->bufs(), h->skey, h->sord, h->soff, h->sval, h->sidx, h->stemp,

@@ -74,6 +74,12 @@ struct Bufs {
     const float *seed_d;
     float *bound;  // forward: [p][n_rows] starting bounds of a seeded step (k_seed_bounds)
     int use_seeds;
+    // the pruned scan (snn_scan.cu): the step's candidates packed [group][column][32];
+    // backward: [group][column] extremes over the group's candidates, and per
+    // feature (mean, min, max, -) of its training column
+    float *xg;
+    float2 *ext;
+    const float4 *fstat;
     int only_if_full;  // scoring kernels return at once unless st->full_scan is set (sorted first step)
 };
 
@@ -100,9 +106,16 @@ bool score_tma_supported(int kmax);  // kernel option 3: k_max <= 64
 cudaError_t launch_score_tma(const Bufs &b, int n_cand, int backward, cudaStream_t s);
 int score_tma_launches(int kmax, int n_cand, int backward);  // kernels one launch_score_tma issues
 // Seeded forward steps: each candidate's starting bound from the seed columns, into b.bound.
-// xrm: n_cols x n_cand floats of scratch (the candidates' columns row-major),
-// or null to take the bounds from part of the seeds (k_seed_bounds).
-cudaError_t launch_seed_bounds(const Bufs &b, int n_cand, float *xrm, cudaStream_t s);
+// packed: b.xg holds the step's candidates (launch_pack_groups).
+cudaError_t launch_seed_bounds(const Bufs &b, int n_cand, cudaStream_t s);
+
+// Pruned scan (snn_scan.cu), k_max <= kScoreMaxK, given starting bounds (forward
+// b.bound, backward b.kth_prev) and the packed candidates b.xg.
+bool scan_supported(int n_cols, int kmax);
+int scan_groups(int n_cand);      // groups of at most 32 candidates
+int scan_group_size(int n_cand);  // candidates of a full group
+cudaError_t launch_pack_groups(const Bufs &b, int n_cand, int backward, cudaStream_t s);
+cudaError_t launch_scan(const Bufs &b, int n_cand, int backward, int max_smem, cudaStream_t s);
 
 // Commit the winner into D (snn_commit.cu); forward commits given seed
 // buffers also keep kSeeds near columns per row for the next step's bounds.
@@ -136,8 +149,9 @@ cudaError_t launch_mode_predict(const Bufs &b, int n_cand, cudaStream_t s);
 cudaError_t launch_losses(const Bufs &b, int n_cand, cudaStream_t s);
 // Per row of D: the largest finite entry (backward; D only shrinks afterwards).
 cudaError_t launch_row_dmax(const Bufs &b, float *dmax, cudaStream_t s);
-// Per-feature training variance (FP64 sums) into var[p], NaN for non-finite columns.
-cudaError_t launch_feature_variance(const Bufs &b, float *var, cudaStream_t s);
+// Per-feature training variance (FP64 sums) into var[p], NaN for non-finite columns; with stat
+// also (mean or 0, smallest, largest, 0) of the column.
+cudaError_t launch_feature_variance(const Bufs &b, float *var, float4 *stat, cudaStream_t s);
 // perm[0..p) = features by ascending var (NaN last, ties by id): the candidate slot order.
 cudaError_t launch_feature_order(const float *var, int p, int *perm, cudaStream_t s);
 cudaError_t launch_force(const Bufs &b, int w, int it, int t, int total_steps, int backward, cudaStream_t s);

@@ -338,25 +338,36 @@ __global__ void k_row_dmax(Bufs b, float *dmax)
 
 // One block per feature: variance of the training column (FP64 sums).  Used
 // only to order candidate slots so that a scoring warp's candidates have
-// distances of similar scale; never part of a result.
-__global__ void k_feature_variance(Bufs b, float *var)
+// distances of similar scale; never part of a result.  stat (backward):
+// (mean, or 0 where it is not finite; smallest; largest; 0) of the column, NaN
+// left out, for the bounds of the pruned scan.
+__global__ void k_feature_variance(Bufs b, float *var, float4 *stat)
 {
     const int j = blockIdx.x;
     const float *x = b.XT + (size_t)j * b.ldc;
     double s1 = 0.0, s2 = 0.0;
+    float lo = INFINITY, hi = -INFINITY;
     for (int i = threadIdx.x; i < b.n_cols; i += blockDim.x) {
-        const double v = x[i];
+        const float f = x[i];
+        const double v = f;
         s1 += v;
         s2 += v * v;
+        lo = fminf(lo, f);
+        hi = fmaxf(hi, f);
     }
     __shared__ double r1[8], r2[8];
+    __shared__ float rlo[8], rhi[8];
     for (int o = 16; o > 0; o >>= 1) {
         s1 += __shfl_xor_sync(0xffffffffu, s1, o);
         s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
     }
     if ((threadIdx.x & 31) == 0) {
         r1[threadIdx.x >> 5] = s1;
         r2[threadIdx.x >> 5] = s2;
+        rlo[threadIdx.x >> 5] = lo;
+        rhi[threadIdx.x >> 5] = hi;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -364,10 +375,13 @@ __global__ void k_feature_variance(Bufs b, float *var)
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
             t1 += r1[w];
             t2 += r2[w];
+            lo = fminf(lo, rlo[w]);
+            hi = fmaxf(hi, rhi[w]);
         }
         const double m = t1 / b.n_cols;
         const double v = t2 / b.n_cols - m * m;
         var[j] = isfinite(v) ? (float)fmax(v, 0.0) : NAN;
+        if (stat) stat[j] = make_float4(isfinite((float)m) ? (float)m : 0.0f, lo, hi, 0.0f);
     }
 }
 
@@ -448,9 +462,9 @@ cudaError_t launch_force(const Bufs &b, int w, int it, int t, int total_steps, i
     return cudaGetLastError();
 }
 
-cudaError_t launch_feature_variance(const Bufs &b, float *var, cudaStream_t s)
+cudaError_t launch_feature_variance(const Bufs &b, float *var, float4 *stat, cudaStream_t s)
 {
-    k_feature_variance<<<b.p, 256, 0, s>>>(b, var);
+    k_feature_variance<<<b.p, 256, 0, s>>>(b, var, stat);
     return cudaGetLastError();
 }
 

@@ -401,45 +401,27 @@ __device__ __forceinline__ float warp_kth(float (&v)[V], int K, int lane)
     return __shfl_sync(kFull, sel, (K - 1) / V);
 }
 
-// xrm[i][slot] = X[cands[slot]][i]: the step's candidate columns, row-major
-// (n_cols x n_cand), through 32 x 32 shared-memory tiles.
-__global__ void __launch_bounds__(256) k_candidates_rowmajor(Bufs b, int n_cand, float *xrm)
-{
-    __shared__ float tile[32][33];
-    if (b.st->done) return;
-    const int i0 = blockIdx.x * 32, s0 = blockIdx.y * 32;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int k = ty; k < 32; k += 8) {
-        const int slot = s0 + k, i = i0 + tx;
-        tile[k][tx] = slot < n_cand && i < b.n_cols ? __ldg(b.XT + (size_t)__ldg(b.cands + slot) * b.ldc + i) : 0.0f;
-    }
-    __syncthreads();
-    for (int k = ty; k < 32; k += 8) {
-        const int i = i0 + k, slot = s0 + tx;
-        if (i < b.n_cols && slot < n_cand) xrm[(size_t)i * n_cand + slot] = tile[tx][k];
-    }
-}
-
 // k_seed_bounds_exact (K <= L <= 16): the bound of each (candidate, scored row)
 // problem is the K-th smallest exact distance d = fl(D + fl((x_r,c - x_i,c)^2))
 // over ALL kSeeds seed columns of the row (see k_seed_bounds for why any K
 // distinct columns bound the final K-th distance).  One warp per row, lane l
-// taking candidate slot l (then l + 32, ...): the L smallest distances seen
+// taking candidate l of each group of the pruned scan in turn: the L smallest distances seen
 // sit sorted in registers (L the list length rounded up to 4, 8, 12 or 16), and each seed column's values for 32 candidates
-// are one contiguous read of xrm.  Seeds are taken in the commit's order;
+// are one contiguous read of the packed candidates xg.  Seeds are taken in the commit's order;
 // a seed whose committed distance already reaches every lane's L-th smallest
 // is skipped (d >= D).
 template <int L>
-__global__ void __launch_bounds__(256) k_seed_bounds_exact(Bufs b, int n_cand, const float *xrm, float *bound)
+__global__ void __launch_bounds__(256) k_seed_bounds_exact(Bufs b, int n_cand, int G, int gs, float *bound)
 {
     if (b.st->done) return;
     const int lane = threadIdx.x & 31;
     const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (r >= b.n_rows) return;  // warp-uniform
     const int K = b.kmax;
-    for (int c0 = 0; c0 < n_cand; c0 += 32) {
-        const int slot = c0 + lane;
-        const bool live = slot < n_cand;
+    for (int g = 0; g < G; ++g) {
+        const int slot = g * gs + lane;
+        const bool live = lane < gs && slot < n_cand;
+        const float *xg = b.xg + (size_t)g * b.ldc * 32 + lane;
         const int c = live ? __ldg(b.cands + slot) : 0;  // the candidate feature
         const float xv = live ? __ldg(b.XV + (size_t)c * b.ldr + r) : 0.0f;
         float l[L];
@@ -456,7 +438,7 @@ __global__ void __launch_bounds__(256) k_seed_bounds_exact(Bufs b, int n_cand, c
                 for (int u = 0; u < 8; ++u) {
                     ii[u] = __shfl_sync(kFull, myi, j8 + u);
                     DD[u] = __shfl_sync(kFull, myd, j8 + u);
-                    xx[u] = live && ii[u] >= 0 ? __ldg(xrm + (size_t)ii[u] * n_cand + slot) : 0.0f;
+                    xx[u] = ii[u] >= 0 ? __ldg(xg + (size_t)ii[u] * 32) : 0.0f;
                 }
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
@@ -490,7 +472,7 @@ __global__ void __launch_bounds__(256) k_seed_bounds_exact(Bufs b, int n_cand, c
 // distances count as +inf.  One warp per row, lane l holding seeds
 // l + 32 j (j < kSeedsPerLane); the gathers of two candidates are issued
 // together, and many warps per SM hide their latency.  Each lane keeps its
-// V smallest values (V = 2 for K <= 16, 4 above), and the K-th smallest of
+// V smallest values (V = 4 up to K = 128, all 8 above), and the K-th smallest of
 // those 32 V values is the bound: a subset of the seeds, so still K distinct
 // columns, and as tight as all of them unless a lane holds more than V of
 // the K nearest.
@@ -1084,19 +1066,16 @@ cudaError_t launch_k(const Bufs &b, int n_cand, int max_smem, cudaStream_t s)
 
 }  // namespace
 
-cudaError_t launch_seed_bounds(const Bufs &b, int n_cand, float *xrm, cudaStream_t s)
+cudaError_t launch_seed_bounds(const Bufs &b, int n_cand, cudaStream_t s)
 {
     const int grid = (b.n_rows + 7) / 8;
-    if (b.kmax <= 16 && xrm) {
-        k_candidates_rowmajor<<<dim3((b.n_cols + 31) / 32, (n_cand + 31) / 32), 256, 0, s>>>(b, n_cand, xrm);
-        if (b.kmax <= 4) k_seed_bounds_exact<4><<<grid, 256, 0, s>>>(b, n_cand, xrm, b.bound);
-        else if (b.kmax <= 8) k_seed_bounds_exact<8><<<grid, 256, 0, s>>>(b, n_cand, xrm, b.bound);
-        else if (b.kmax <= 12) k_seed_bounds_exact<12><<<grid, 256, 0, s>>>(b, n_cand, xrm, b.bound);
-        else k_seed_bounds_exact<16><<<grid, 256, 0, s>>>(b, n_cand, xrm, b.bound);
-        return cudaGetLastError();
-    }
-    if (b.kmax > 16) k_seed_bounds<4><<<grid, 256, 0, s>>>(b, n_cand, b.bound);
-    else k_seed_bounds<2><<<grid, 256, 0, s>>>(b, n_cand, b.bound);
+    const int G = scan_groups(n_cand), gs = scan_group_size(n_cand);
+    if (b.kmax <= 4) k_seed_bounds_exact<4><<<grid, 256, 0, s>>>(b, n_cand, G, gs, b.bound);
+    else if (b.kmax <= 8) k_seed_bounds_exact<8><<<grid, 256, 0, s>>>(b, n_cand, G, gs, b.bound);
+    else if (b.kmax <= 12) k_seed_bounds_exact<12><<<grid, 256, 0, s>>>(b, n_cand, G, gs, b.bound);
+    else if (b.kmax <= 16) k_seed_bounds_exact<16><<<grid, 256, 0, s>>>(b, n_cand, G, gs, b.bound);
+    else if (b.kmax <= 128) k_seed_bounds<4><<<grid, 256, 0, s>>>(b, n_cand, b.bound);
+    else k_seed_bounds<8><<<grid, 256, 0, s>>>(b, n_cand, b.bound);
     return cudaGetLastError();
 }
 

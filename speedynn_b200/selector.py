@@ -145,7 +145,7 @@ class Selector:
         return cands, pred
 
     def set_kernel(self, which):
-        """Scoring kernel: 0 automatic, 1 rows per lane (any k), 3 TMA-fed row tiles (k <= 64)."""
+        """Scoring kernel: 0 automatic (pruned scan where a step has bounds), 1 rows per lane (any k), 3 TMA-fed row tiles (k <= 64)."""
         check(_lib.lib().snn_set_option(self._h, _lib.SNN_OPT_KERNEL, int(which)))
 
     def set_sorted_start(self, enable):
@@ -153,8 +153,8 @@ class Selector:
         check(_lib.lib().snn_set_option(self._h, _lib.SNN_OPT_SORTED_START, int(bool(enable))))
 
     def set_seed_step(self, step):
-        """First forward step whose starting bounds come from seed columns (default 2, 3 for k > 16;
-        a large value turns seeded steps off).  Results do not depend on it."""
+        """First forward step whose starting bounds come from seed columns (default 2 for holdout
+        problems with k <= 64, else 1; a large value turns seeded steps off).  Results do not depend on it."""
         check(_lib.lib().snn_set_option(self._h, _lib.SNN_OPT_SEED_STEP, int(step)))
 
     def set_counters(self, enable):
