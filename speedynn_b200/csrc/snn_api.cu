@@ -48,9 +48,8 @@ int fail(int code, const char *fmt, ...)
 
 inline int round_up(int x, int m) { return (x + m - 1) / m * m; }
 
-struct EventPair {
-    cudaEvent_t a = nullptr, b = nullptr;
-};
+using snn::Block;
+using snn::EventPair;
 
 }  // namespace
 
@@ -88,7 +87,7 @@ struct snn_handle {
     float *kth_prev = nullptr;     // backward: last step's k-th distances [p][n_rows]
     float *dmax = nullptr;         // backward: per row, the largest finite entry of the full D
     bool prev_ok = false;          // kth_prev holds the previous step's values
-    int inject_stall = -1;         // fault injection (see dev_alloc): stage to withhold once
+    int inject_stall = -1;         // fault injection (see carve): stage to withhold once
     int inject_launch = -1;        // fault injection: greedy step whose launch fails once
     bool extra_losses() const { return !(loss_ids.size() == 1 && loss_ids[0] == 0); }
     State *st = nullptr;
@@ -123,11 +122,16 @@ struct snn_handle {
     int host_step = 0;  // steps issued since the last reset
     // timing
     bool step_events = true;  // per-step CUDA events (off for batch problems: only total_ev is read)
-    bool arena = false;       // device buffers are sub-allocations of a batch arena (never freed one by one)
+    bool arena = false;       // device buffers are sub-allocations of a batch arena, which outlives the handle
+    Block block;              // the handle's buffers, its stream and spare events (not with an arena)
+    Block model_block;        // snn_set_model's loss buffers
+    Block nn_block;           // kept neighbour lists
+    bool fresh = false;       // nothing has touched the state or D since the last reset
     std::vector<EventPair> score_ev, commit_ev;
     EventPair total_ev;
     EventPair setup_ev;  // the last reset's initial distance matrix (full distance or empty)
     bool setup_timed = false;
+    bool total_timed = false;  // total_ev was recorded since the last reset_timing
     int n_score = 0, n_commit = 0, n_launch = 0;
 
     Bufs bufs() const
@@ -191,70 +195,69 @@ namespace {
 //                             of stage N, so its bounded waits run out (SNN_ERR_TIMEOUT)
 thread_local int t_fail_alloc = 0;  // countdown to the injected allocation failure, 0 = off
 
-// Bump allocator over one device allocation: while a batch creates and loads
-// the problems of a wave on this thread, their buffers are carved from it
-// (one cudaMalloc per batch run instead of a score per problem; cudaFree
-// also waits for the whole device).  256-byte aligned sub-allocations.
+// Bump allocator over one device allocation, 256-byte aligned: a handle's
+// buffers come from one block (snn_blocks.cu), those of a batch wave's problems
+// from one allocation for the wave.  Without a base it only counts.
 struct Arena {
     char *base = nullptr;
     size_t cap = 0, used = 0;
 };
-thread_local Arena *t_arena = nullptr;
+thread_local Arena *t_arena = nullptr;  // a batch's, while it creates and loads its problems on this thread
 
 template <typename T>
-int dev_alloc(T **p, size_t n, const char *what)
+int carve(Arena &a, T **p, size_t n, const char *what)
 {
     *p = nullptr;
-    if (t_fail_alloc > 0 && --t_fail_alloc == 0) return fail(SNN_ERR_NOMEM, "injected failure of the allocation of %s", what);
+    if (a.base && t_fail_alloc > 0 && --t_fail_alloc == 0)
+        return fail(SNN_ERR_NOMEM, "injected failure of the allocation of %s", what);
     if (n == 0) n = 1;
-    if (t_arena) {
-        const size_t off = (t_arena->used + 255) & ~(size_t)255;
-        const size_t bytes = n * sizeof(T);
-        if (off > t_arena->cap || bytes > t_arena->cap - off)
-            return fail(SNN_ERR_NOMEM, "batch arena full at %s (%zu bytes)", what, bytes);
-        *p = reinterpret_cast<T *>(t_arena->base + off);
-        t_arena->used = off + bytes;
-        return SNN_OK;
-    }
-    cudaError_t e = cudaMalloc((void **)p, n * sizeof(T));
-    if (e != cudaSuccess) {
-        *p = nullptr;
-        cudaGetLastError();
-        return fail(e == cudaErrorMemoryAllocation ? SNN_ERR_NOMEM : SNN_ERR_CUDA,
-                    "cudaMalloc of %s (%zu bytes) failed: %s", what, n * sizeof(T), cudaGetErrorString(e));
-    }
+    const size_t off = (a.used + 255) & ~(size_t)255;
+    const size_t bytes = n * sizeof(T);
+    if (off > a.cap || bytes > a.cap - off) return fail(SNN_ERR_NOMEM, "no room for %s (%zu bytes)", what, bytes);
+    if (a.base) *p = reinterpret_cast<T *>(a.base + off);
+    a.used = off + bytes;
     return SNN_OK;
+}
+
+// Carve what `take` asks for from the batch's arena, or from a block acquired for it.
+template <typename F>
+int take_buffers(snn_handle *h, Block &block, const char *what, F take)
+{
+    if (t_arena) return take(*t_arena);
+    Arena count;
+    count.cap = ~(size_t)0 / 2;
+    if (int rc = take(count)) return rc;
+    const cudaError_t e = snn::block_acquire(h->device, count.used, &block);
+    if (e != cudaSuccess)
+        return fail(e == cudaErrorMemoryAllocation ? SNN_ERR_NOMEM : SNN_ERR_CUDA, "device memory for %s (%zu bytes): %s", what,
+                    count.used, cudaGetErrorString(e));
+    Arena a;
+    a.base = block.base;
+    a.cap = block.bytes;
+    return take(a);
 }
 
 void free_all(snn_handle *h)
 {
     cudaSetDevice(h->device);
-    if (!h->arena) {  // an arena's buffers are freed by its owner
-        void *ptrs[] = {h->XT, h->cv ? nullptr : h->XV, h->yc, h->cv ? nullptr : h->yr, h->D, h->pred, h->rmse32,
-                        h->err, h->stage, h->rmse64, h->err64, h->kv, h->cands, h->prev_cands, h->mask, h->order,
-                        h->stepk, h->st, h->nn_idx, h->nn_dist, h->seeds, h->seed_d, h->sbound, h->sval, h->skey, h->sidx,
-                        h->sord, h->soff, h->stemp, h->walked, h->perm, h->fvar,
-                        h->d_loss_ids, h->lossval, h->err_all, h->kth_prev, h->dmax, h->fcount, h->xg, h->ext, h->fstat};
-        for (void *q : ptrs)
-            if (q) cudaFree(q);
-    }
-    for (auto &e : h->score_ev) {
-        if (e.a) cudaEventDestroy(e.a);
-        if (e.b) cudaEventDestroy(e.b);
-    }
-    for (auto &e : h->commit_ev) {
-        if (e.a) cudaEventDestroy(e.a);
-        if (e.b) cudaEventDestroy(e.b);
-    }
-    if (h->total_ev.a) cudaEventDestroy(h->total_ev.a);
-    if (h->total_ev.b) cudaEventDestroy(h->total_ev.b);
-    if (h->setup_ev.a) cudaEventDestroy(h->setup_ev.a);
-    if (h->setup_ev.b) cudaEventDestroy(h->setup_ev.b);
-    if (h->stream) cudaStreamDestroy(h->stream);
+    const bool idle = !h->stream || cudaStreamSynchronize(h->stream) == cudaSuccess;
+    std::vector<EventPair> &ev = h->block.events;
+    ev.insert(ev.end(), h->score_ev.begin(), h->score_ev.end());
+    ev.insert(ev.end(), h->commit_ev.begin(), h->commit_ev.end());
+    ev.push_back(h->total_ev);
+    ev.push_back(h->setup_ev);
+    h->block.stream = h->stream;  // with an arena the block holds no memory, and its stream and events go
+    snn::block_release(h->model_block, idle);
+    snn::block_release(h->nn_block, idle);
+    snn::block_release(h->block, idle);
 }
 
-int make_pair(EventPair &e)
+int make_pair(snn_handle *h, EventPair &e)
 {
+    while (!(e.a && e.b) && !h->block.events.empty()) {  // an earlier handle's
+        e = h->block.events.back();
+        h->block.events.pop_back();
+    }
     if (!e.a) SNN_CUDA(cudaEventCreate(&e.a));
     if (!e.b) SNN_CUDA(cudaEventCreate(&e.b));
     return SNN_OK;
@@ -269,10 +272,11 @@ int check_device(int device)
         return fail(SNN_ERR_CUDA, "no CUDA device available (%s)", cudaGetErrorString(e));
     }
     if (device < 0 || device >= n) return fail(SNN_ERR_ARG, "device %d out of range (%d devices)", device, n);
-    cudaDeviceProp prop;
-    SNN_CUDA(cudaGetDeviceProperties(&prop, device));
-    if (prop.major != 10) return fail(SNN_ERR_CUDA, "device %d is sm_%d%d; this library is built for sm_100a", device,
-                                      prop.major, prop.minor);
+    // two attributes: the whole property structure takes the driver 1 to 30 ms
+    int major = 0, minor = 0;
+    SNN_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
+    SNN_CUDA(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device));
+    if (major != 10) return fail(SNN_ERR_CUDA, "device %d is sm_%d%d; this library is built for sm_100a", device, major, minor);
     return SNN_OK;
 }
 
@@ -314,6 +318,7 @@ bool sorted_step(const snn_handle *h, int t)
 // Issue one greedy step (no synchronisation).
 int issue_step(snn_handle *h, int t)
 {
+    h->fresh = false;
     Bufs b = h->bufs();
     const int n_cand = h->p - t;  // forward: p - t unselected; backward: p - t still selected
     const int backward = h->desc.backward;
@@ -322,7 +327,7 @@ int issue_step(snn_handle *h, int t)
     if (h->step_events) {
         if ((int)h->score_ev.size() <= h->n_score) h->score_ev.resize(h->n_score + 1);
         se = &h->score_ev[h->n_score];
-        if (int rc = make_pair(*se)) return rc;
+        if (int rc = make_pair(h, *se)) return rc;
         SNN_CUDA(cudaEventRecord(se->a, h->stream));
     }
     if (t == h->inject_launch) {
@@ -382,7 +387,7 @@ int issue_step(snn_handle *h, int t)
         if (h->step_events) {
             if ((int)h->commit_ev.size() <= h->n_commit) h->commit_ev.resize(h->n_commit + 1);
             ce = &h->commit_ev[h->n_commit];
-            if (int rc = make_pair(*ce)) return rc;
+            if (int rc = make_pair(h, *ce)) return rc;
             SNN_CUDA(cudaEventRecord(ce->a, h->stream));
         }
         const bool sd = seeds_for_step(h, t + 1);
@@ -399,6 +404,7 @@ int issue_step(snn_handle *h, int t)
 
 int issue_reset(snn_handle *h)
 {
+    h->fresh = false;
     h->prev_ok = false;
     h->seeds_ok = false;
     h->last_ncand = 0;
@@ -406,7 +412,7 @@ int issue_reset(snn_handle *h)
     SNN_CUDA(snn::launch_reset_state(b, h->desc.backward, h->total_steps, h->stream));
     h->setup_timed = h->step_events;
     if (h->setup_timed) {
-        if (int rc = make_pair(h->setup_ev)) return rc;
+        if (int rc = make_pair(h, h->setup_ev)) return rc;
         SNN_CUDA(cudaEventRecord(h->setup_ev.a, h->stream));
     }
     if (h->desc.backward) {
@@ -419,6 +425,7 @@ int issue_reset(snn_handle *h)
     if (h->setup_timed) SNN_CUDA(cudaEventRecord(h->setup_ev.b, h->stream));
     h->n_launch += 2;
     h->host_step = 0;
+    h->fresh = true;
     return SNN_OK;
 }
 
@@ -432,6 +439,7 @@ int read_state(snn_handle *h, State *s)
 void reset_timing(snn_handle *h)
 {
     h->n_score = h->n_commit = h->n_launch = 0;
+    h->total_timed = false;
     if (h->fcount) cudaMemsetAsync(h->fcount, 0, 3 * sizeof(unsigned long long), h->stream);
 }
 
@@ -489,6 +497,63 @@ static size_t handle_bytes(const snn_desc *d, int kmax)
     return sizeof(float) * f + ((size_t)1 << 20);
 }
 
+// Every buffer of a handle, in one order for counting and for carving.
+static int carve_buffers(snn_handle *h, Arena &a)
+{
+    int rc = SNN_OK;
+    const int backward = h->desc.backward;
+    const size_t p = (size_t)h->p;
+    if ((rc = carve(a, &h->XT, p * h->ldc, "X_train"))) return rc;
+    if ((rc = carve(a, &h->yc, (size_t)h->n_cols, "y_train"))) return rc;
+    if (h->cv) {
+        h->XV = h->XT;
+        h->yr = h->yc;
+    } else {
+        if ((rc = carve(a, &h->XV, p * h->ldr, "X_val"))) return rc;
+        if ((rc = carve(a, &h->yr, (size_t)h->n_rows, "y_val"))) return rc;
+    }
+    if ((rc = carve(a, &h->D, (size_t)h->n_rows * h->ldc, "distance matrix"))) return rc;
+    if ((rc = carve(a, &h->pred, p * h->nk * h->n_rows, "predictions"))) return rc;
+    if ((rc = carve(a, &h->rmse32, p * h->nk, "errors"))) return rc;
+    if ((rc = carve(a, &h->rmse64, p * h->nk, "errors64"))) return rc;
+    // the results, read back in one copy (snn_get_results)
+    if ((rc = carve(a, &h->err64, p, "step errors64"))) return rc;
+    if ((rc = carve(a, &h->err, p, "step errors"))) return rc;
+    if ((rc = carve(a, &h->mask, p, "mask"))) return rc;
+    if ((rc = carve(a, &h->order, p, "ordering"))) return rc;
+    if ((rc = carve(a, &h->stepk, p, "best k"))) return rc;
+    if ((rc = carve(a, &h->st, 1, "state"))) return rc;
+    if ((rc = carve(a, &h->kv, (size_t)h->nk, "k_vals"))) return rc;
+    if ((rc = carve(a, &h->cands, p, "candidates"))) return rc;
+    if ((rc = carve(a, &h->prev_cands, p, "candidates"))) return rc;
+    if ((rc = carve(a, &h->perm, p, "feature order"))) return rc;
+    if (backward && (rc = carve(a, &h->kth_prev, p * (size_t)h->n_rows, "k-th distances"))) return rc;
+    if (backward && (rc = carve(a, &h->dmax, (size_t)h->n_rows, "row maxima"))) return rc;
+    if ((rc = carve(a, &h->fvar, p, "feature variances"))) return rc;
+    if ((rc = carve(a, &h->fcount, 3, "filter counters"))) return rc;
+    if (!backward) {
+        if ((rc = carve(a, &h->seeds, (size_t)h->n_rows * snn::kSeeds, "seed columns"))) return rc;
+        if ((rc = carve(a, &h->seed_d, (size_t)h->n_rows * snn::kSeeds, "seed distances"))) return rc;
+        if ((rc = carve(a, &h->sbound, p * h->n_rows, "seed bounds"))) return rc;
+    }
+    const size_t groups = (p + 31) / 32;
+    if ((rc = carve(a, &h->xg, groups * h->ldc * 32, "packed candidates"))) return rc;
+    if (backward && (rc = carve(a, &h->ext, groups * h->ldc, "column extremes"))) return rc;
+    if (backward && (rc = carve(a, &h->fstat, p, "feature ranges"))) return rc;
+    if (!backward && !h->cv) {
+        const size_t pl = p * h->ldc;
+        if ((rc = carve(a, &h->sval, pl, "sorted values"))) return rc;
+        // the sort's keys at load, then the second step's candidate values in sorted order
+        if ((rc = carve(a, &h->skey, pl, "sort keys"))) return rc;
+        if ((rc = carve(a, &h->sidx, pl, "sorted indices"))) return rc;
+        if ((rc = carve(a, &h->sord, pl, "sort values"))) return rc;
+        if ((rc = carve(a, &h->soff, 2 * p, "sort offsets"))) return rc;
+        if ((rc = carve(a, &h->stemp, h->stemp_bytes, "sort workspace"))) return rc;
+        if ((rc = carve(a, &h->walked, 1, "walk counter"))) return rc;
+    }
+    return carve(a, &h->stage, (size_t)std::max(h->n_rows, h->n_cols) * p, "staging");
+}
+
 SNN_API int snn_create(const snn_desc *d, snn_handle **out)
 {
     g_err.clear();
@@ -539,65 +604,18 @@ SNN_API int snn_create(const snn_desc *d, snn_handle **out)
     h->plan = snn::plan_score(kmax, d->p, max_smem);
     if (h->plan.cc == 0)
         return bail(fail(SNN_ERR_UNSUPPORTED, "k_max=%d is above the supported maximum of %d", kmax, snn::kScoreMaxK));
-    if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess)
+    if (!h->desc.backward && !cv) h->stemp_bytes = snn::sort_temp_bytes(h->p, h->ldc);
+    if ((rc = take_buffers(h, h->block, "a problem", [&](Arena &a) { return carve_buffers(h, a); }))) return bail(rc);
+    h->stream = h->block.stream;
+    if (!h->stream && cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess)
         return bail(fail(SNN_ERR_CUDA, "cudaStreamCreate failed"));
-
-    const size_t p = (size_t)h->p;
-    if ((rc = dev_alloc(&h->XT, p * h->ldc, "X_train"))) return bail(rc);
-    if ((rc = dev_alloc(&h->yc, (size_t)h->n_cols, "y_train"))) return bail(rc);
-    if (cv) {
-        h->XV = h->XT;
-        h->yr = h->yc;
-    } else {
-        if ((rc = dev_alloc(&h->XV, p * h->ldr, "X_val"))) return bail(rc);
-        if ((rc = dev_alloc(&h->yr, (size_t)h->n_rows, "y_val"))) return bail(rc);
-    }
-    if ((rc = dev_alloc(&h->D, (size_t)h->n_rows * h->ldc, "distance matrix"))) return bail(rc);
-    if ((rc = dev_alloc(&h->pred, p * h->nk * h->n_rows, "predictions"))) return bail(rc);
-    if ((rc = dev_alloc(&h->rmse32, p * h->nk, "errors"))) return bail(rc);
-    if ((rc = dev_alloc(&h->rmse64, p * h->nk, "errors64"))) return bail(rc);
-    if ((rc = dev_alloc(&h->err, p, "step errors"))) return bail(rc);
-    if ((rc = dev_alloc(&h->err64, p, "step errors64"))) return bail(rc);
-    if ((rc = dev_alloc(&h->kv, (size_t)h->nk, "k_vals"))) return bail(rc);
-    if ((rc = dev_alloc(&h->cands, p, "candidates"))) return bail(rc);
-    if ((rc = dev_alloc(&h->prev_cands, p, "candidates"))) return bail(rc);
-    if ((rc = dev_alloc(&h->perm, p, "feature order"))) return bail(rc);
-    if (d->backward && (rc = dev_alloc(&h->kth_prev, p * (size_t)h->n_rows, "k-th distances"))) return bail(rc);
-    if (d->backward && (rc = dev_alloc(&h->dmax, (size_t)h->n_rows, "row maxima"))) return bail(rc);
-    if ((rc = dev_alloc(&h->fvar, p, "feature variances"))) return bail(rc);
-    if ((rc = dev_alloc(&h->mask, p, "mask"))) return bail(rc);
-    if ((rc = dev_alloc(&h->order, p, "ordering"))) return bail(rc);
-    if ((rc = dev_alloc(&h->stepk, p, "best k"))) return bail(rc);
-    if ((rc = dev_alloc(&h->st, 1, "state"))) return bail(rc);
-    if ((rc = dev_alloc(&h->fcount, 3, "filter counters"))) return bail(rc);
-    if (!d->backward) {
-        if ((rc = dev_alloc(&h->seeds, (size_t)h->n_rows * snn::kSeeds, "seed columns"))) return bail(rc);
-        if ((rc = dev_alloc(&h->seed_d, (size_t)h->n_rows * snn::kSeeds, "seed distances"))) return bail(rc);
-        if ((rc = dev_alloc(&h->sbound, p * h->n_rows, "seed bounds"))) return bail(rc);
-    }
-    const size_t groups = (p + 31) / 32;
-    if ((rc = dev_alloc(&h->xg, groups * h->ldc * 32, "packed candidates"))) return bail(rc);
-    if (d->backward && (rc = dev_alloc(&h->ext, groups * h->ldc, "column extremes"))) return bail(rc);
-    if (d->backward && (rc = dev_alloc(&h->fstat, p, "feature ranges"))) return bail(rc);
-    if (!d->backward && !cv) {
-        const size_t pl = p * h->ldc;
-        if ((rc = dev_alloc(&h->sval, pl, "sorted values"))) return bail(rc);
-        // the sort's keys at load, then the second step's candidate values in sorted order
-        if ((rc = dev_alloc(&h->skey, pl, "sort keys"))) return bail(rc);
-        if ((rc = dev_alloc(&h->sidx, pl, "sorted indices"))) return bail(rc);
-        if ((rc = dev_alloc(&h->sord, pl, "sort values"))) return bail(rc);
-        if ((rc = dev_alloc(&h->soff, 2 * p, "sort offsets"))) return bail(rc);
-        h->stemp_bytes = snn::sort_temp_bytes(h->p, h->ldc);
-        if ((rc = dev_alloc(&h->stemp, h->stemp_bytes, "sort workspace"))) return bail(rc);
-        if ((rc = dev_alloc(&h->walked, 1, "walk counter"))) return bail(rc);
-    }
     // On the handle's stream, so every kernel that reads k_vals comes after it
     // (the source lives as long as the handle).  A cudaMemcpy here would run on
     // the legacy stream, which does not order the handle's non-blocking stream,
     // and from pageable memory it may return before its DMA lands.
     if (cudaMemcpyAsync(h->kv, h->kvals.data(), sizeof(int) * h->nk, cudaMemcpyHostToDevice, h->stream) != cudaSuccess)
         return bail(fail(SNN_ERR_CUDA, "copy of k_vals failed"));
-    if (make_pair(h->total_ev)) return bail(SNN_ERR_CUDA);
+    if (make_pair(h, h->total_ev)) return bail(SNN_ERR_CUDA);
     t_fail_alloc = 0;
     *out = h;
     return SNN_OK;
@@ -608,10 +626,6 @@ static int load_matrix(snn_handle *h, const float *X, int n, float *XT, int ld, 
     const size_t bytes = sizeof(float) * (size_t)n * h->p;
     const float *src = X;
     if (!device_src) {
-        if (!h->stage) {
-            size_t n_stage = (size_t)std::max(h->n_rows, h->n_cols) * h->p;
-            if (int rc = dev_alloc(&h->stage, n_stage, "staging")) return rc;
-        }
         SNN_CUDA(cudaMemcpyAsync(h->stage, X, bytes, cudaMemcpyHostToDevice, h->stream));
         src = h->stage;
     }
@@ -678,12 +692,15 @@ SNN_API int snn_run(snn_handle *h)
     SNN_CUDA(cudaSetDevice(h->device));
     reset_timing(h);
     SNN_CUDA(cudaEventRecord(h->total_ev.a, h->stream));
-    // every run is a complete selection from the initial distance matrix
-    if (int rc = issue_reset(h)) return rc;
+    // every run is a complete selection from the initial distance matrix, which
+    // is still there right after a load or a reset (fwd-64k: 1.5 ms, bwd-50k 21 ms)
+    if (!h->fresh)
+        if (int rc = issue_reset(h)) return rc;
     for (int t = 0; t < h->total_steps; ++t)
         if (int rc = issue_step(h, t)) return rc;
     h->host_step = h->total_steps;
     SNN_CUDA(cudaEventRecord(h->total_ev.b, h->stream));
+    h->total_timed = true;
     State s;
     if (int rc = read_state(h, &s)) return rc;
     if (s.error == snn::kErrTimeout) return fail(SNN_ERR_TIMEOUT, "a device pipeline wait timed out at step %d", s.step);
@@ -705,6 +722,7 @@ SNN_API int snn_step(snn_handle *h)
     SNN_CUDA(cudaEventRecord(h->total_ev.a, h->stream));
     if (int rc = issue_step(h, h->host_step)) return rc;
     SNN_CUDA(cudaEventRecord(h->total_ev.b, h->stream));
+    h->total_timed = true;
     h->host_step++;
     if (int rc = read_state(h, &s)) return rc;
     if (s.error == snn::kErrTimeout) return fail(SNN_ERR_TIMEOUT, "a device pipeline wait timed out at step %d", s.step);
@@ -727,8 +745,10 @@ SNN_API int snn_commit_sequence(snn_handle *h, const int *seq, int n)
     }
     SNN_CUDA(cudaSetDevice(h->device));
     reset_timing(h);
-    if (int rc = issue_reset(h)) return rc;
+    if (!h->fresh)
+        if (int rc = issue_reset(h)) return rc;
     const Bufs b = h->bufs();
+    if (n > 0) h->fresh = false;
     for (int t = 0; t < n; ++t) {
         const int it = h->desc.backward ? h->p - 1 - t : t;
         SNN_CUDA(snn::launch_force(b, seq[t], it, t, h->total_steps, h->desc.backward, h->stream));
@@ -748,16 +768,37 @@ SNN_API int snn_get_results(snn_handle *h, int *ordering, int *mask, float *erro
     if (!h) return fail(SNN_ERR_ARG, "null handle");
     SNN_CUDA(cudaSetDevice(h->device));
     const size_t p = (size_t)h->p;
-    if (ordering) SNN_CUDA(cudaMemcpyAsync(ordering, h->order, p * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    if (mask) SNN_CUDA(cudaMemcpyAsync(mask, h->mask, p * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    if (errors) SNN_CUDA(cudaMemcpyAsync(errors, h->err, p * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
-    if (errors64) SNN_CUDA(cudaMemcpyAsync(errors64, h->err64, p * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    if (step_best_k) SNN_CUDA(cudaMemcpyAsync(step_best_k, h->stepk, p * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    // err64 ... st lie together (carve_buffers): one copy, then the parts
+    const char *base = reinterpret_cast<const char *>(h->err64);
+    std::vector<char> host((size_t)(reinterpret_cast<const char *>(h->st + 1) - base));
+    SNN_CUDA(cudaMemcpyAsync(host.data(), base, host.size(), cudaMemcpyDeviceToHost, h->stream));
+    SNN_CUDA(cudaStreamSynchronize(h->stream));
+    auto part = [&](void *dst, const void *src, size_t bytes) {
+        if (dst) memcpy(dst, host.data() + (reinterpret_cast<const char *>(src) - base), bytes);
+    };
+    part(ordering, h->order, p * sizeof(int));
+    part(mask, h->mask, p * sizeof(int));
+    part(errors, h->err, p * sizeof(float));
+    part(errors64, h->err64, p * sizeof(double));
+    part(step_best_k, h->stepk, p * sizeof(int));
     State s;
-    if (int rc = read_state(h, &s)) return rc;
+    part(&s, h->st, sizeof s);
     if (best_k) *best_k = s.best_k_last;
     if (num_final) *num_final = s.num_final;
     return SNN_OK;
+}
+
+// The kept neighbour lists of a step, taken once.
+static int take_lists(snn_handle *h)
+{
+    if (h->nn_idx) return SNN_OK;
+    const size_t n = (size_t)h->p * h->n_rows * h->kmax;
+    const int rc = take_buffers(h, h->nn_block, "neighbour lists", [&](Arena &a) {
+        const int e = carve(a, &h->nn_idx, n, "neighbour indices");
+        return e ? e : carve(a, &h->nn_dist, n, "neighbour distances");
+    });
+    if (rc) h->nn_idx = nullptr, h->nn_dist = nullptr;
+    return rc;
 }
 
 SNN_API int snn_set_model(snn_handle *h, const int *loss_ids, int n_losses, int model_type)
@@ -770,30 +811,26 @@ SNN_API int snn_set_model(snn_handle *h, const int *loss_ids, int n_losses, int 
     if (model_type != 0 && model_type != 1) return fail(SNN_ERR_ARG, "model_type %d is not 0 or 1", model_type);
     SNN_CUDA(cudaSetDevice(h->device));
     SNN_CUDA(cudaStreamSynchronize(h->stream));
-    if (!h->arena) {  // an arena's sub-allocations are freed with the arena
-        cudaFree(h->d_loss_ids);
-        cudaFree(h->lossval);
-        cudaFree(h->err_all);
-    }
+    snn::block_release(h->model_block, true);  // an arena's sub-allocations are freed with the arena
     h->d_loss_ids = nullptr;
     h->lossval = h->err_all = nullptr;
     h->loss_ids.assign(loss_ids, loss_ids + n_losses);
     h->model = model_type;
     const size_t nl = (size_t)n_losses, p = (size_t)h->p;
     if (h->extra_losses()) {
-        if (int rc = dev_alloc(&h->d_loss_ids, nl, "loss ids")) return rc;
-        if (int rc = dev_alloc(&h->lossval, nl * p * h->nk, "losses")) return rc;
-        if (int rc = dev_alloc(&h->err_all, nl * p, "losses per step")) return rc;
+        if (int rc = take_buffers(h, h->model_block, "losses", [&](Arena &a) {
+                int e = carve(a, &h->d_loss_ids, nl, "loss ids");
+                if (!e) e = carve(a, &h->lossval, nl * p * h->nk, "losses");
+                return e ? e : carve(a, &h->err_all, nl * p, "losses per step");
+            }))
+            return rc;
         // on the handle's stream (see the k_vals copy in snn_create); the wait lets
         // the caller reuse loss_ids at once
         SNN_CUDA(cudaMemcpyAsync(h->d_loss_ids, h->loss_ids.data(), sizeof(int) * nl, cudaMemcpyHostToDevice, h->stream));
         SNN_CUDA(cudaStreamSynchronize(h->stream));
     }
-    if (model_type == 1 && !h->nn_idx) {
-        const size_t n = p * h->n_rows * h->kmax;
-        if (int rc = dev_alloc(&h->nn_idx, n, "neighbour indices")) return rc;
-        if (int rc = dev_alloc(&h->nn_dist, n, "neighbour distances")) return rc;
-    }
+    if (model_type == 1)
+        if (int rc = take_lists(h)) return rc;
     if (h->loaded) {
         if (int rc = issue_reset(h)) return rc;
         SNN_CUDA(cudaStreamSynchronize(h->stream));
@@ -822,11 +859,8 @@ SNN_API int snn_keep_neighbours(snn_handle *h, int enable)
     g_err.clear();
     if (!h) return fail(SNN_ERR_ARG, "null handle");
     SNN_CUDA(cudaSetDevice(h->device));
-    if (enable && !h->nn_idx) {
-        const size_t n = (size_t)h->p * h->n_rows * h->kmax;
-        if (int rc = dev_alloc(&h->nn_idx, n, "neighbour indices")) return rc;
-        if (int rc = dev_alloc(&h->nn_dist, n, "neighbour distances")) return rc;
-    }
+    if (enable)
+        if (int rc = take_lists(h)) return rc;
     h->keep_nn = enable != 0;
     h->nn_ncand = 0;
     return SNN_OK;
@@ -936,7 +970,7 @@ SNN_API int snn_get_timing(snn_handle *h, double *score_ms, int *score_launches,
         c += ms;
     }
     float tot = 0.f;
-    if (h->n_launch > 0) {
+    if (h->total_timed) {
         cudaError_t e = cudaEventElapsedTime(&tot, h->total_ev.a, h->total_ev.b);
         if (e != cudaSuccess) {
             cudaGetLastError();
@@ -1080,6 +1114,7 @@ int issue_batch_problem(snn_handle *h)
         if (int rc = issue_step(h, t)) return rc;
     h->host_step = h->total_steps;
     SNN_CUDA(cudaEventRecord(h->total_ev.b, h->stream));
+    h->total_timed = true;
     return SNN_OK;
 }
 
@@ -1206,12 +1241,18 @@ SNN_API int snn_batch_run(snn_batch *B)
             const size_t reserve = std::max<size_t>((size_t)1 << 30, tot / 50);
             budget = fr > reserve ? fr - reserve : 0;
         }
-        // the wave's buffers come from one device allocation of the budget
-        // (without it, from cudaMalloc per buffer)
+        // the wave's buffers come from one device allocation: what the problems
+        // that fit the budget need, not the whole budget (mapping 160 GB takes
+        // 60 to 180 ms and unmapping 80); without it, from a block per problem
         // (a wave always admits its first problem, whatever the budget)
-        int kmax0 = 0;
-        validate_desc(&B->prob[i].desc, &kmax0);
-        const size_t cap = std::max(budget, handle_bytes(&B->prob[i].desc, kmax0) + model_bytes(B->prob[i], kmax0));
+        size_t cap = 0;
+        for (int k = i; k < n && B->prob[k].desc.device == dev; ++k) {
+            int kmax = 0;
+            validate_desc(&B->prob[k].desc, &kmax);
+            const size_t need = handle_bytes(&B->prob[k].desc, kmax) + model_bytes(B->prob[k], kmax);
+            if (cap && cap + need > budget) break;
+            cap += need;
+        }
         Arena arena;
         void *abase = nullptr;
         if (cudaMalloc(&abase, cap) == cudaSuccess) {

@@ -6,7 +6,30 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <vector>
+
 namespace snn {
+
+struct EventPair {
+    cudaEvent_t a = nullptr, b = nullptr;
+};
+
+// A device allocation that buffers are carved from (snn_blocks.cu), with the
+// stream and timing events of the handle that had it last.
+struct Block {
+    char *base = nullptr;
+    size_t bytes = 0;
+    int device = 0;
+    unsigned long long id = 0;  // the driver's id of the allocation
+    cudaStream_t stream = nullptr;
+    std::vector<EventPair> events;
+};
+// A block of at least `bytes` bytes on the current device, a spare one if there is one.
+cudaError_t block_acquire(int device, size_t bytes, Block *out);
+// Give a block back: kept as a spare if it is small and nothing uses it any more (idle), else freed.
+void block_release(Block &b, bool idle);
+// Free a device's spare blocks.
+void blocks_trim(int device);
 
 // Selection state kept on the device so that a whole greedy step (score ->
 // reduce -> select -> commit) runs without a host round trip.
