@@ -14,7 +14,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libspeedynn_b200.so")
 SOURCES = ["snn_kernels.cu", "snn_score.cu", "snn_commit.cu", "snn_sorted.cu", "snn_score_tma.cu", "snn_scan.cu", "snn_model.cu", "snn_noalloc.cu", "snn_blocks.cu", "snn_api.cu", "snn_compat.cpp"]
-HEADERS = ["snn_internal.h"]
+HEADERS = ["snn_internal.h", "snn_packed.cuh"]
 
 NVCC_FLAGS = [
     "-O3", "-std=c++17", "-lineinfo",

@@ -106,6 +106,7 @@ struct snn_handle {
     float *xg = nullptr;          // pruned scan: packed candidates [ceil(p / 32)][ldc][32]
     float2 *ext = nullptr;        // backward: [ceil(p / 32)][ldc] column extremes
     float4 *fstat = nullptr;      // backward: per-feature mean and range
+    int *walk = nullptr, *n_walk = nullptr;  // forward holdout: problems left to k_walk, and how many
     bool sorted_start = true;     // SNN_OPT_SORTED_START
     bool seeds_ok = false;        // seeds hold the current D's seed columns
     int seed_step = 2;            // SNN_OPT_SEED_STEP: first forward step scored from seed bounds (set at create)
@@ -181,6 +182,10 @@ struct snn_handle {
         b.xg = xg;
         b.ext = ext;
         b.fstat = fstat;
+        b.walk = walk;
+        b.n_walk = n_walk;
+        b.sval = sval;
+        b.sidx = sidx;
         b.only_if_full = 0;
         return b;
     }
@@ -297,13 +302,22 @@ bool seeds_for_step(const snn_handle *h, int t)
     return !h->desc.backward && h->seeds && h->kernel != 1 && t >= h->seed_step;
 }
 
-// The automatic choice scores a step by the pruned scan (snn_scan.cu) once it
-// has starting bounds: forward from seed columns, backward from the previous
-// step's k-th distances.  The filter counters and the injected stall belong to
-// the TMA-fed scorer, so a step that wants them takes that one.
-bool scan_step(const snn_handle *h)
+// How the automatic choice scores step t by the pruned scan (snn_scan.cu): the
+// seeding mode, or -1 for another scorer.  Backward steps start from the
+// previous step's k-th distances, the first one (and the first after a warm
+// start) from seed columns that the scan finds itself (25,003 x 12,502 x 120:
+// 3.9 ms, dense 10.2); forward steps from the commit's seed columns.  With
+// nothing committed every column is open, which the scan takes only where its
+// shorter chain of work beats the dense scorer's rate (step 1 of a 3000-row CV
+// problem: 0.38 ms, dense 0.58).  The filter counters and the injected stall
+// belong to the TMA-fed scorer, so a step that wants them takes that one.
+constexpr int kScanAllCols = 4096;
+int scan_seeding(const snn_handle *h, int t, bool seeded)
 {
-    return h->kernel == 0 && snn::scan_supported(h->n_cols, h->kmax) && !(h->count_filter || h->inject_stall >= 0) && (h->desc.backward ? h->prev_ok : h->seeds_ok);
+    if (h->kernel != 0 || h->count_filter || h->inject_stall >= 0) return -1;
+    if (h->desc.backward) return h->prev_ok ? snn::kNoSeeds : snn::kOwnSeeds;
+    if (seeded) return snn::kGivenSeeds;
+    return t == 0 && h->n_cols <= kScanAllCols ? snn::kOwnSeeds : -1;
 }
 
 // The first two forward steps of a holdout problem run from sorted feature
@@ -342,14 +356,20 @@ int issue_step(snn_handle *h, int t)
     }
     const bool seeded = !backward && h->seeds_ok && seeds_for_step(h, t);
     bool prev = false;  // this step writes every candidate's k-th distances (backward)
-    const bool scan = !b.only_if_full && scan_step(h) && (backward || seeded);
-    if (scan || (seeded && use_tma(h))) {
+    const int seeding = b.only_if_full ? -1 : scan_seeding(h, t, seeded);
+    const bool scan = seeding >= 0;
+    const bool dense_seeded = !scan && seeded && use_tma(h);
+    if (scan || dense_seeded) {
         SNN_CUDA(snn::launch_pack_groups(b, n_cand, backward, h->stream));
-        if (seeded) SNN_CUDA(snn::launch_seed_bounds(b, n_cand, h->stream));
-        h->n_launch += seeded ? 2 : 1;
+        if (dense_seeded) SNN_CUDA(snn::launch_seed_bounds(b, n_cand, h->stream));
+        h->n_launch += dense_seeded ? 2 : 1;
     }
     if (scan) {
-        SNN_CUDA(snn::launch_scan(b, n_cand, backward, h->max_smem, h->stream));
+        SNN_CUDA(snn::launch_scan(b, n_cand, backward, seeding, h->max_smem, h->stream));
+        if (snn::scan_leaves_walks(b, n_cand, backward)) {
+            SNN_CUDA(snn::launch_walk(b, h->stream));
+            h->n_launch += 1;
+        }
         prev = backward;
     } else if (use_tma(h)) {
         b.use_prev = backward && h->prev_ok ? 1 : 0;
@@ -489,7 +509,7 @@ static size_t handle_bytes(const snn_desc *d, int kmax)
     size_t f = p * ldc + n_rows * ldc + p * (size_t)d->num_k_vals * n_rows + std::max(n_rows, n_cols) * p +
                n_rows * M + n_cols + n_rows;
     // sorted feature columns of the first forward step and the sort's buffers
-    if (!d->backward && !cv) f += 4 * p * ldc + 2 * p + snn::sort_temp_bytes(d->p, (int)ldc) / sizeof(float) + 1;
+    if (!d->backward && !cv) f += p * n_rows + 4 * p * ldc + 2 * p + snn::sort_temp_bytes(d->p, (int)ldc) / sizeof(float) + 1;
     if (d->backward) f += p * n_rows + n_rows;  // kth_prev, dmax
     const size_t groups = (p + 31) / 32;         // packed candidates of the pruned scan, backward: their extremes
     f += groups * ldc * 32 + (d->backward ? 2 * groups * ldc + 4 * p : 0);
@@ -550,6 +570,8 @@ static int carve_buffers(snn_handle *h, Arena &a)
         if ((rc = carve(a, &h->soff, 2 * p, "sort offsets"))) return rc;
         if ((rc = carve(a, &h->stemp, h->stemp_bytes, "sort workspace"))) return rc;
         if ((rc = carve(a, &h->walked, 1, "walk counter"))) return rc;
+        if ((rc = carve(a, &h->walk, p * h->n_rows, "walks"))) return rc;
+        if ((rc = carve(a, &h->n_walk, 1, "walk count"))) return rc;
     }
     return carve(a, &h->stage, (size_t)std::max(h->n_rows, h->n_cols) * p, "staging");
 }

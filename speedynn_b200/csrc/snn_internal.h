@@ -103,6 +103,13 @@ struct Bufs {
     float *xg;
     float2 *ext;
     const float4 *fstat;
+    // forward problems that the scan leaves to k_walk: slot * n_rows + r of
+    // each, how many, and every feature's sorted values with their columns
+    // ([p][ldc], null where nothing is sorted)
+    int *walk;
+    int *n_walk;
+    const float *sval;
+    const int *sidx;
     int only_if_full;  // scoring kernels return at once unless st->full_scan is set (sorted first step)
 };
 
@@ -132,13 +139,18 @@ int score_tma_launches(int kmax, int n_cand, int backward);  // kernels one laun
 // packed: b.xg holds the step's candidates (launch_pack_groups).
 cudaError_t launch_seed_bounds(const Bufs &b, int n_cand, cudaStream_t s);
 
-// Pruned scan (snn_scan.cu), k_max <= kScoreMaxK, given starting bounds (forward
-// b.bound, backward b.kth_prev) and the packed candidates b.xg.
-bool scan_supported(int n_cols, int kmax);
-int scan_groups(int n_cand);      // groups of at most 32 candidates
-int scan_group_size(int n_cand);  // candidates of a full group
+// Pruned scan (snn_scan.cu), k_max <= kScoreMaxK, given the packed candidates
+// b.xg.  Where its starting bounds come from: nowhere else than b.kth_prev
+// (backward, after a scored step), the seed columns b.seeds that the commit
+// kept, or seed columns that the kernel finds itself.
+enum { kNoSeeds = 0, kGivenSeeds = 1, kOwnSeeds = 2 };
+inline int scan_groups(int n_cand) { return (n_cand + 31) / 32; }  // groups of at most 32 candidates
+inline int scan_group_size(int n_cand) { return (n_cand + scan_groups(n_cand) - 1) / scan_groups(n_cand); }  // of a full group
 cudaError_t launch_pack_groups(const Bufs &b, int n_cand, int backward, cudaStream_t s);
-cudaError_t launch_scan(const Bufs &b, int n_cand, int backward, int max_smem, cudaStream_t s);
+// May leave problems in b.walk for launch_walk (scan_leaves_walks).
+cudaError_t launch_scan(const Bufs &b, int n_cand, int backward, int seeding, int max_smem, cudaStream_t s);
+bool scan_leaves_walks(const Bufs &b, int n_cand, int backward);
+cudaError_t launch_walk(const Bufs &b, cudaStream_t s);
 
 // Commit the winner into D (snn_commit.cu); forward commits given seed
 // buffers also keep kSeeds near columns per row for the next step's bounds.

@@ -15,22 +15,24 @@
 // bound by the FP32 pipe on the other 99 %.
 //
 // One warp per (scored row, group of up to 32 candidates), lane = candidate:
+//   * starting bounds: backward the previous step's k-th distances; forward from
+//     the row's 256 seed columns, for k <= 16 by group minima, above (and where
+//     nobody kept seeds) by putting the seed columns into the lists first;
 //   * the warp streams its row of D, 512 columns at a time, and queues the
 //     columns that any of its candidates may still take (the sign of D - H, H
 //     the group's largest bound, which falls as the lists fill);
-//   * queued columns are taken eight at a time, their candidate values gathered
+//   * queued columns are taken in batches, their candidate values gathered
 //     together from `xg`, the candidates packed [group][column][32] (one aligned
 //     128-byte line per column and group, so a gather is one full-width load);
 //     every lane forms its candidate's exact distance and appends it to its
 //     own buffer in shared memory if it may enter the list;
-//   * when a lane's buffer is nearly full, all lanes empty theirs together into
+//   * when a lane's buffer is half full, all lanes empty theirs together into
 //     their lists, heaps of k_max (distance, column) keys in shared memory.  The
 //     keys are ordered by distance, then column, which is the reference's
 //     stable rule in whatever order the columns arrive;
-//   * forward, a row that is an outlier in some features leaves those
-//     candidates' bounds far above the others'.  Such candidates ("wide") are
-//     kept out of H and scanned with lane = column instead; the split minimises
-//     the cost estimated from 256 sampled columns;
+//   * forward, a row that is an outlier in a feature leaves that candidate's
+//     bound far above the others'.  Such problems are left to k_walk
+//     (snn_sorted.cu), the split by the cost estimated from sampled columns;
 //   * backward, H takes each candidate's largest possible s on the row; a
 //     queued column is tested once more, with the group's extreme values in
 //     that column (`ext`), before it is gathered.
@@ -38,29 +40,34 @@
 // with the insertion unrolled at every use the kernel waited for instructions
 // 80 % of the time.
 //
-// What bounds it: instruction issue (59 % of the slots on a 16,384 x 8,192 step
-// with 14 warps per SM, each waiting for its own chain) well above the D stream
-// (fwd-64k: 3 ms per late step, 1.3 ms of it the read of D).  Scoring of a whole
-// fwd-64k selection 293 -> 80 ms, a step of bwd-50k's quarter size 7.0 -> 1.4 ms,
-// a k = 150 step of 8,192 x 4,096 x 19 130 -> 8 ms.
+// What bounds it: instruction issue (55 to 60 % of the slots; the rest is each
+// warp's own chain) well above the D stream: fwd-64k 3.3 ms per late step, 1.3 ms
+// of it the read of D.  Scoring of a whole fwd-64k selection 293 -> 71 ms
+// (80 with the bounds in a kernel of their own and the outliers scanned here
+// with lane = column, 128 columns per exposed load), a backward step of 25,003
+// x 12,502 7.0 -> 1.0 ms, a k = 50 step of 50,021 x 24,989 57 -> 13 ms, a
+// k = 150 step of 8,192 x 4,096 x 19 130 -> 6 ms.
 #include <float.h>
 #include <math.h>
 #include <stdint.h>
 
 #include "snn_internal.h"
+#include "snn_packed.cuh"
 
 namespace snn {
 
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kUnroll = 4;             // float4 loads of D per lane and pass of the loop
-constexpr int kCols = 128 * kUnroll;   // columns per pass of the loop
-constexpr int kQueue = 1024;           // entries of a warp's column queue (a power of two, above kCols + kBatch)
-constexpr int kBatch = 8;              // queued columns gathered together
-constexpr int kBuf = 16;               // distances a lane buffers before they enter its heap
-constexpr int kTagShift = 26;          // queue entry: column, and above it 1 + lane of a wide candidate (0: the others)
-constexpr int kWarps = 1;              // warps per block: they finish at different times
+constexpr int kUnroll = 4;            // float4 loads of D per lane and pass of the loop
+constexpr int kCols = 128 * kUnroll;  // columns per pass of the loop
+constexpr int kQueue = 256;           // entries of a warp's column queues (a power of two, kSeeds at least)
+constexpr float kCap = 0x1.fffffcp+127f;  // largest distance that can enter a list (items at FLT_MAX never do)
+// Instructions of a warp, for choosing who walks (k_scan): a queued column, the
+// start of a walk, a column of it (1.6 instructions, but its gather of D fetches
+// 64 bytes from memory, worth more; fwd-64k 120 ms a selection at 4, 118 at 9).
+constexpr float kQueueCost = 14.0f, kWalkStart = 3000.0f, kWalkCost = 8.0f;
+static_assert(kQueue >= kSeeds && kQueue >= 128 + 16 + 32, "room for a pass's columns");
 
 // Order-preserving signed key of a float (no NaN), and back.
 __device__ __forceinline__ int fkey(float v)
@@ -70,12 +77,21 @@ __device__ __forceinline__ int fkey(float v)
 }
 __device__ __forceinline__ float fkey_inv(int k) { return __int_as_float(k ^ ((k >> 31) & 0x7fffffff)); }
 
-// List keys: (distance, column) as one unsigned 64-bit number.
+// List keys: (distance, column) as one unsigned 64-bit number.  Forward
+// distances are >= +0, so their bits order like the values; backward ones may
+// be negative.
+template <bool BWD>
 __device__ __forceinline__ unsigned long long pack_key(float d, int col)
 {
-    return ((unsigned long long)((unsigned)fkey(d) ^ 0x80000000u) << 32) | (unsigned)col;
+    const unsigned u = BWD ? (unsigned)fkey(d) ^ 0x80000000u : __float_as_uint(d);
+    return ((unsigned long long)u << 32) | (unsigned)col;
 }
-__device__ __forceinline__ float key_dist(unsigned long long k) { return fkey_inv((int)((unsigned)(k >> 32) ^ 0x80000000u)); }
+template <bool BWD>
+__device__ __forceinline__ float key_dist(unsigned long long k)
+{
+    const unsigned u = (unsigned)(k >> 32);
+    return BWD ? fkey_inv((int)(u ^ 0x80000000u)) : __uint_as_float(u);
+}
 
 // Replace the root of the lane's max-heap h[0], h[32], ... (n entries) by key.
 __device__ __forceinline__ void sift_down(unsigned long long *h, int n, unsigned long long key)
@@ -99,26 +115,42 @@ __device__ __forceinline__ void sift_down(unsigned long long *h, int n, unsigned
     h[i * 32] = key;
 }
 
-// Shared memory of a warp: heaps and buffers of 32 lanes, column queue(s).
-size_t warp_smem(int K, bool bwd)
+// Shared memory of a warp: heaps and buffers (two batches) of 32 lanes, one or two lists of columns.
+size_t warp_smem(int K, int batch, bool aux)
 {
-    return sizeof(unsigned long long) * 32 * (size_t)(K + kBuf) + sizeof(int) * (size_t)kQueue * (bwd ? 2 : 1);
+    return sizeof(unsigned long long) * 32 * (size_t)(K + 2 * batch) + sizeof(int) * (size_t)kQueue * (aux ? 2 : 1);
 }
 
-template <bool BWD>
-__global__ void __launch_bounds__(32 * kWarps, 20) k_scan(Bufs b, int n_cand, int G, int gs, int wsmem, int wide_cost)
+__device__ __forceinline__ unsigned sign_in(unsigned m, float v) { return __funnelshift_l(__float_as_uint(v), m, 1); }
+
+// What a kernel instance does before it scans the row (SEED): nothing
+// (backward, bounds from the last step); bound every candidate's k-th distance
+// by SEED group minima over the row's seed columns; or put the seed columns
+// into the heaps.
+constexpr int kSeedNone = 0, kSeedHeap = -1;
+
+// kBatch queued columns are gathered together, and a lane buffers up to twice
+// as many keys before they enter its heap.  Large problems take batches of 4 at
+// 64 registers and 28 warps per SM, which hide the gathers for one another
+// (fwd-64k 118.0 ms a selection; batches of 8 with 20 warps 122.7, with the
+// loads of one batch under the work of the last one at 16 warps 139.6);
+// problems of at most one such wave of warps, whose time is the chain of
+// gathers of one warp, take batches of 16.
+constexpr int kBatchMany = 4, kBatchFew = 16, kWarpsMany = 28;
+
+template <bool BWD, int SEED, int kBatch>
+__global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_scan(Bufs b, int n_cand, int G, int gs, int walks, int own)
 {
+    constexpr int kBuf = 2 * kBatch;
     extern __shared__ __align__(16) unsigned char smraw[];
     if (b.st->done) return;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int gw = blockIdx.x * (blockDim.x >> 5) + w;
-    const int r = gw / G, g = gw % G;
-    if (r >= b.n_rows) return;  // warp-uniform; nothing below synchronises the block
+    const int lane = threadIdx.x;  // blocks of one warp: warps finish at different times
+    const int r = blockIdx.x / G, g = blockIdx.x % G;
     const int K = b.kmax;
-    unsigned long long *heap = reinterpret_cast<unsigned long long *>(smraw + (size_t)w * wsmem) + lane;
+    unsigned long long *heap = reinterpret_cast<unsigned long long *>(smraw) + lane;
     unsigned long long *buf = heap + (size_t)K * 32;
-    int *queue = reinterpret_cast<int *>(smraw + (size_t)w * wsmem + sizeof(unsigned long long) * 32 * (size_t)(K + kBuf));
-    int *wait = queue + kQueue;  // backward: columns before the second test
+    int *queue = reinterpret_cast<int *>(smraw + sizeof(unsigned long long) * 32 * (size_t)(K + kBuf));
+    int *aux = queue + kQueue;  // backward: columns before the second test; kSeedHeap: the lanes' seed columns
 
     const int slot = g * gs + lane;
     const bool live = lane < gs && slot < n_cand;
@@ -129,24 +161,122 @@ __global__ void __launch_bounds__(32 * kWarps, 20) k_scan(Bufs b, int n_cand, in
     const size_t cr = (size_t)c * b.n_rows + r;
     const float *xg = b.xg + (size_t)g * b.ldc * 32 + lane;
     const float *Dr = b.D + (size_t)r * b.ldc;
-
-    // lim: distances above it cannot enter the lane's list.  The list starts as K
-    // sentinels at the (inclusive) bound, ordered after every column; those left
-    // at the end are padding.
-    float lim = -INFINITY;
-    if (act) {
-        lim = BWD ? b.kth_prev[cr] : b.bound[cr];
-        if (!(lim < FLT_MAX)) lim = 0x1.fffffcp+127f;  // items at FLT_MAX never enter
-    }
-    for (int j = 0; j < K; ++j) heap[j * 32] = pack_key(lim, -1);
-
     const float4 *row = reinterpret_cast<const float4 *>(Dr);
     const int n4 = b.ldc >> 2;
-    float4 nxt[kUnroll];
+
+    // lim: distances above it cannot enter the lane's list.
+    float lim = act ? kCap : -INFINITY;
+    if (BWD && SEED == kSeedNone && act) lim = fminf(b.kth_prev[cr], kCap);
+    if constexpr (SEED > 0) {
+        // Any k distinct columns bound the k-th distance.  The minimum over each
+        // group of 8 (k <= 8) or 4 seed columns belongs to another column, and the
+        // k-th smallest of the 32 or 64 minima is nearly as tight as that of all 256
+        // columns (for k = 10: the 4.2 % quantile of their distances instead of 3.9 %)
+        // at an eighth or a quarter of the list insertions.
+        constexpr int P = SEED <= 8 ? 8 : 4;
+        float L[SEED];  // ascending; the first SEED - K entries -inf, so the k-th is the last
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-        const int q = u * 32 + lane;
-        nxt[u] = q < n4 ? __ldg(row + q) : make_float4(INFINITY, INFINITY, INFINITY, INFINITY);
+        for (int j = 0; j < SEED; ++j) L[j] = j < SEED - K ? -INFINITY : INFINITY;
+        const int *seeds = b.seeds + (size_t)r * kSeeds + lane;
+        const float *seed_d = b.seed_d + (size_t)r * kSeeds + lane;
+        int ni = __ldg(seeds);
+        float nd = __ldg(seed_d);
+#pragma unroll 1
+        for (int j0 = 0; j0 < kSeeds; j0 += 32) {
+            const int myi = ni;
+            const float myd = nd;
+            if (j0 + 32 < kSeeds) {
+                ni = __ldg(seeds + j0 + 32);
+                nd = __ldg(seed_d + j0 + 32);
+            }
+#pragma unroll 1
+            for (int l0 = 0; l0 < 32; l0 += 8) {
+                float D[8], x[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    D[i] = __shfl_sync(kFull, myd, l0 + i);  // +inf for an absent column (-1)
+                    x[i] = __ldg(xg + (size_t)max(__shfl_sync(kFull, myi, l0 + i), 0) * 32);
+                }
+#pragma unroll
+                for (int i = 0; i < 8; i += P) {
+                    float v = INFINITY;
+#pragma unroll
+                    for (int u = 0; u < P; ++u) {
+                        const float t = __fsub_rn(xv, x[i + u]);
+                        v = fminf(v, __fadd_rn(D[i + u], __fmul_rn(t, t)));  // a NaN is left out
+                    }
+                    if (__any_sync(kFull, v < L[SEED - 1])) {
+#pragma unroll
+                        for (int q = SEED - 1; q > 0; --q) L[q] = fminf(L[q], fmaxf(L[q - 1], v));
+                        L[0] = fminf(L[0], v);
+                    }
+                }
+            }
+        }
+        if (act) lim = fminf(L[SEED - 1], kCap);
+    }
+
+    // The list starts as K sentinels at the (inclusive) bound, ordered after every
+    // column; those left at the end are padding.
+    for (int j = 0; j < K; ++j) heap[j * 32] = pack_key<BWD>(lim, -1);
+
+    int qh = 0, qn = 0;  // queue: first entry, entries
+    // kSeedHeap: the seed columns go through the queue before the row's others; the
+    // lane keeps its own (the commit and this kernel give each lane the same
+    // columns), ascending, to leave them out afterwards.
+    int nseed = 0;  // the lane's seed columns not yet passed, the last ones at aux[32 * i + lane]
+    if constexpr (SEED == kSeedHeap) {
+        int si[kSeedsPerLane];
+        if (!own) {
+#pragma unroll
+            for (int j = 0; j < kSeedsPerLane; ++j) si[j] = __ldg(b.seeds + (size_t)r * kSeeds + j * 32 + lane);
+        } else {
+            // nobody kept them: the lane's kSeedsPerLane nearest, from a pass of its own
+            float sv[kSeedsPerLane];
+#pragma unroll
+            for (int j = 0; j < kSeedsPerLane; ++j) {
+                sv[j] = INFINITY;
+                si[j] = -1;
+            }
+#pragma unroll 1
+            for (int q = lane; q < n4; q += 32) {
+                float4 d = __ldg(row + q);
+#pragma unroll 1
+                for (int e = 0; e < 4; ++e) {
+                    const float v = d.x;
+                    d = make_float4(d.y, d.z, d.w, 0.0f);
+                    if (v < sv[kSeedsPerLane - 1]) {
+#pragma unroll
+                        for (int j = kSeedsPerLane - 1; j > 0; --j) {
+                            const bool here = v < sv[j], before = v < sv[j - 1];
+                            si[j] = before ? si[j - 1] : here ? 4 * q + e : si[j];
+                            sv[j] = before ? sv[j - 1] : here ? v : sv[j];
+                        }
+                        if (v < sv[0]) {
+                            sv[0] = v;
+                            si[0] = 4 * q + e;
+                        }
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kSeedsPerLane; ++j) {  // nearest first
+            const unsigned m = __ballot_sync(kFull, si[j] >= 0);
+            if (si[j] >= 0) queue[qn + __popc(m & ((1u << lane) - 1u))] = si[j];
+            qn += __popc(m);
+            nseed += si[j] >= 0 ? 1 : 0;
+        }
+#pragma unroll
+        for (int i = 1; i < kSeedsPerLane; ++i)  // ascending, absent ones (-1) first
+#pragma unroll
+            for (int j = i; j > 0; --j) {
+                const int lo = min(si[j - 1], si[j]), hi = max(si[j - 1], si[j]);
+                si[j - 1] = lo;
+                si[j] = hi;
+            }
+#pragma unroll
+        for (int j = 0; j < kSeedsPerLane; ++j) aux[32 * j + lane] = si[j];
     }
 
     // Backward: each candidate's largest possible square on this row and the
@@ -167,123 +297,132 @@ __global__ void __launch_bounds__(32 * kWarps, 20) k_scan(Bufs b, int n_cand, in
         }
     }
 
-    // Forward: which candidates are scanned with lane = column (wide): the cut
-    // with the least estimated cost.  A wide candidate costs wide_cost sampled
-    // columns, any other the sampled columns within its bound, the group the
-    // most of them (launch_dir has the figures).
-    unsigned wide = 0u;
-    if constexpr (!BWD) {
-        if (wide_cost > 0) {
-            float smp[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) smp[i] = __ldg(Dr + (size_t)i * (b.n_cols / 8) + lane);
-            int cnt = 0;  // sampled columns within the lane's bound
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll 4
-                for (int l = 0; l < 32; ++l) cnt += __shfl_sync(kFull, smp[i], l) <= lim ? 1 : 0;
-            int above = 0;  // candidates with more columns than this lane's
-#pragma unroll 4
-            for (int l = 0; l < 32; ++l) above += __shfl_sync(kFull, cnt, l) > cnt ? 1 : 0;
-            const int best = __reduce_min_sync(kFull, ((wide_cost * above + cnt) << 9) | cnt);  // cost, then the cut
-            wide = __ballot_sync(kFull, cnt > (best & 511));
-        }
-    }
-    const bool reg = !((wide >> lane) & 1u);
-
     // No column with D >= H can enter a list of the queue's candidates: forward
     // d >= D; backward d <= lim means D - s < nextafter(lim) exactly (rounding is
     // monotone), and s <= smax.  kmx: the same for the second test.
-    float H;
+    float H = 0.0f;
     auto update_H = [&] {
         if constexpr (BWD) {
             const float up = nextafterf(lim, INFINITY);
             H = __int_as_float(__reduce_max_sync(kFull, __float_as_int(fmaxf(__fadd_ru(up, smax), 0.0f))));
             kmx = fkey_inv(__reduce_max_sync(kFull, fkey(up)));
         } else {
-            H = __int_as_float(__reduce_max_sync(kFull, reg ? __float_as_int(fmaxf(lim, 0.0f)) : 0) + 1);
+            H = __int_as_float(__reduce_max_sync(kFull, __float_as_int(fmaxf(lim, 0.0f))) + 1);
         }
     };
+    unsigned wide = 0u;  // forward: candidates left to k_walk, their lim -inf here
+    auto choose_walks = [&] {
+        // The split with the least estimated cost, from 128 sampled columns (64 for
+        // the candidates' own squares): a queued column costs the group kQueueCost
+        // instructions, a walk kWalkStart and kWalkCost for each column whose square
+        // is within the candidate's bound.
+        int cd = 0, cs = 0;  // sampled columns with D, with the square within the lane's bound
+#pragma unroll 1
+        for (int i = 0; i < 4; ++i) {
+            const int j0 = i * (b.n_cols / 4);
+            const float smp = __ldg(Dr + j0 + lane);
+#pragma unroll 8
+            for (int l = 0; l < 32; ++l) cd += __shfl_sync(kFull, smp, l) <= lim ? 1 : 0;
+#pragma unroll 8
+            for (int l = 0; l < 16; ++l) {
+                const float t = xv - __ldg(xg + (size_t)(j0 + l) * 32);
+                cs += t * t <= lim ? 1 : 0;
+            }
+        }
+        const float n = (float)b.n_cols;
+        const int walk = (int)(kWalkStart + kWalkCost / 64.0f * n * (float)cs);
+        int cost = (int)(kQueueCost / 128.0f * n * (float)cd);  // if the candidates with more columns walk
+#pragma unroll 4
+        for (int l = 0; l < 32; ++l) {
+            const int wl = __shfl_sync(kFull, walk, l), cl = __shfl_sync(kFull, cd, l);
+            cost += cl > cd ? wl : 0;
+        }
+        const int best = __reduce_min_sync(kFull, cost);
+        const int cut = __reduce_min_sync(kFull, cost == best ? cd : 999);
+        wide = __ballot_sync(kFull, cd > cut);
+        if (wide) {
+            int at = 0;
+            if (lane == 0) at = atomicAdd(b.n_walk, __popc(wide));
+            at = __shfl_sync(kFull, at, 0) + __popc(wide & ((1u << lane) - 1u));
+            if ((wide >> lane) & 1u) {
+                b.walk[at] = slot * b.n_rows + r;
+                b.bound[cr] = lim;
+                lim = -INFINITY;
+            }
+        }
+    };
+
+    int nb = 0;  // the lane's buffered keys
+    int ah = 0, an = 0;  // backward: columns that wait for the second test (aux)
+    constexpr int q_first = SEED == kSeedHeap ? -kCols : 0;  // a pass for the seed columns first
+    if constexpr (!BWD && SEED != kSeedHeap) {
+        if (walks) choose_walks();
+    }
     update_H();
-
-    // Each lane appends the columns of its 16-bit mask (bit 4u + e: column
-    // q0 + 128 u + 4 lane + e), in no particular order.
-    auto push = [&](int *q, int tail, unsigned m16, int q0, int tag) {
-        int n = 0;
-        for (unsigned any = __ballot_sync(kFull, m16 != 0u); any; any = __ballot_sync(kFull, m16 != 0u)) {
-            if (m16) {
-                const int i = __ffs(m16) - 1;
-                m16 &= m16 - 1;
-                q[(tail + n + __popc(any & ((1u << lane) - 1u))) & (kQueue - 1)] =
-                    (q0 + 128 * (i >> 2) + 4 * lane + (i & 3)) | tag;
+    float4 nxt[kUnroll];
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+        const int q = u * 32 + lane;
+        nxt[u] = q < n4 ? __ldg(row + q) : make_float4(INFINITY, INFINITY, INFINITY, INFINITY);
+    }
+    for (int q0 = q_first;; q0 += kCols) {
+        const bool last = q0 >= b.ldc;  // no columns left: empty the queues
+        const bool drainall = last || q0 < 0;
+        unsigned m16 = 0u;  // bit 4u + e: this lane's column q0 + 128 u + 4 lane + e has D < H
+        if (SEED != kSeedHeap || q0 >= 0) {
+            // the sign of D - H, first column lowest
+            const float2 nH = make_float2(-H, -H);
+#pragma unroll
+            for (int u = kUnroll - 1; u >= 0; --u) {
+                const float2 hi = add2(make_float2(nxt[u].z, nxt[u].w), nH), lo = add2(make_float2(nxt[u].x, nxt[u].y), nH);
+                m16 = sign_in(sign_in(sign_in(sign_in(m16, hi.y), hi.x), lo.y), lo.x);
             }
-            n += __popc(any);
-        }
-        return n;
-    };
-
-    int qh = 0, qn = 0;  // queue: first entry, entries
-    int ah = 0, an = 0;  // backward: columns that wait for the second test
-    int nb = 0;          // the lane's buffered distances
-    for (int q0 = 0;; q0 += kCols) {
-        const bool last = q0 >= b.ldc;  // no columns left: empty the queues and buffers
-        float4 cur[kUnroll];
 #pragma unroll
-        for (int u = 0; u < kUnroll; ++u) {
-            cur[u] = nxt[u];
-            const int q = (q0 >> 2) + (kUnroll + u) * 32 + lane;
-            nxt[u] = q < n4 ? __ldg(row + q) : make_float4(INFINITY, INFINITY, INFINITY, INFINITY);
-        }
-        unsigned todo = wide;
-        for (int ph = -1;;) {  // -1: the columns of the group; then one wide candidate after the other
-            if (ph < 0) {
-                unsigned m16 = 0u;  // sign bits of D - H, first column lowest
-#pragma unroll
-                for (int u = kUnroll - 1; u >= 0; --u) {
-                    m16 = __funnelshift_l(__float_as_uint(__fsub_rn(cur[u].w, H)), m16, 1);
-                    m16 = __funnelshift_l(__float_as_uint(__fsub_rn(cur[u].z, H)), m16, 1);
-                    m16 = __funnelshift_l(__float_as_uint(__fsub_rn(cur[u].y, H)), m16, 1);
-                    m16 = __funnelshift_l(__float_as_uint(__fsub_rn(cur[u].x, H)), m16, 1);
-                }
-                if (q0 + kCols > b.ldc) {  // past the row
-#pragma unroll
-                    for (int u = 0; u < kUnroll; ++u)
-                        if (q0 + 128 * u + 4 * lane >= b.ldc) m16 &= ~(15u << (4 * u));
-                }
-                if constexpr (BWD) an += push(wait, ah + an, m16, q0, 0);
-                else qn += push(queue, qh + qn, m16, q0, 0);
-            } else if constexpr (!BWD) {
-                const float kw = __shfl_sync(kFull, lim, ph), xl = __shfl_sync(kFull, xv, ph);
-                const float4 *xc = reinterpret_cast<const float4 *>(b.XT + (size_t)__shfl_sync(kFull, c, ph) * b.ldc);
-                float4 x[kUnroll];
-#pragma unroll
-                for (int u = 0; u < kUnroll; ++u) {
-                    const int q = (q0 >> 2) + u * 32 + lane;
-                    x[u] = q < n4 ? __ldg(xc + q) : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-                unsigned m16 = 0u;
-#pragma unroll
-                for (int u = 0; u < kUnroll; ++u) {
-                    const float t0 = __fsub_rn(xl, x[u].x), t1 = __fsub_rn(xl, x[u].y), t2 = __fsub_rn(xl, x[u].z),
-                                t3 = __fsub_rn(xl, x[u].w);
-                    m16 |= __fadd_rn(cur[u].x, __fmul_rn(t0, t0)) <= kw ? 1u << (4 * u) : 0u;
-                    m16 |= __fadd_rn(cur[u].y, __fmul_rn(t1, t1)) <= kw ? 2u << (4 * u) : 0u;
-                    m16 |= __fadd_rn(cur[u].z, __fmul_rn(t2, t2)) <= kw ? 4u << (4 * u) : 0u;
-                    m16 |= __fadd_rn(cur[u].w, __fmul_rn(t3, t3)) <= kw ? 8u << (4 * u) : 0u;
-                }
-                // past the row the sums are +inf and never at or below kw
-                qn += push(queue, qh + qn, m16, q0, (int)((unsigned)(ph + 1) << kTagShift));
+            for (int u = 0; u < kUnroll; ++u) {
+                const int q = (q0 >> 2) + (kUnroll + u) * 32 + lane;
+                nxt[u] = q < n4 ? __ldg(row + q) : make_float4(INFINITY, INFINITY, INFINITY, INFINITY);
             }
+            if (q0 + kCols > b.ldc) {  // past the row
+#pragma unroll
+                for (int u = 0; u < kUnroll; ++u)
+                    if (q0 + 128 * u + 4 * lane >= b.ldc) m16 &= ~(15u << (4 * u));
+            }
+            if constexpr (SEED == kSeedHeap) {
+                while (nseed > 0) {
+                    const int i = aux[32 * (kSeedsPerLane - nseed) + lane] - q0;
+                    if (i >= kCols) break;
+                    m16 &= ~(1u << (4 * (i >> 7) + (i & 3)));
+                    --nseed;
+                }
+            }
+        }
+        // Rarely more columns than the queue has room for: then 128 at a time.
+        const int step = __reduce_add_sync(kFull, __popc(m16)) > kQueue - kBatch - 32 ? 4 : 16;
+        for (int part = 0; part < 16; part += step) {
+            // each lane appends its columns, in no particular order
+            unsigned mp = (m16 >> part) & ((1u << step) - 1u);
+            for (unsigned any = __ballot_sync(kFull, mp != 0u); any; any = __ballot_sync(kFull, mp != 0u)) {
+                if (mp) {
+                    const int i = __ffs(mp) - 1 + part;
+                    mp &= mp - 1;
+                    const int at = __popc(any & ((1u << lane) - 1u));
+                    const int col = q0 + 128 * (i >> 2) + 4 * lane + (i & 3);
+                    if constexpr (BWD && SEED == kSeedNone) aux[(ah + an + at) & (kQueue - 1)] = col;
+                    else queue[(qh + qn + at) & (kQueue - 1)] = col;
+                }
+                if constexpr (BWD && SEED == kSeedNone) an += __popc(any);
+                else qn += __popc(any);
+            }
+            __syncwarp();
             for (;;) {
-                if constexpr (BWD) {
+                if constexpr (BWD && SEED == kSeedNone) {
                     if (an >= (last ? 1 : 32)) {
                         // Second test, lane = column: an s of this column is at most U^2, U the
                         // larger of the two extreme differences (rounded up), so an entry needs
                         // D - fl(U^2) < nextafter(lim) for some candidate, and its rounding <= kmx.
-                        __syncwarp();
                         const int n = min(an, 32);
                         const bool in = lane < n;
-                        const int col = in ? wait[(ah + lane) & (kQueue - 1)] : 0;
+                        const int col = in ? aux[(ah + lane) & (kQueue - 1)] : 0;
                         const float D = __ldg(Dr + col);
                         const float2 x = __ldg(b.ext + (size_t)g * b.ldc + col);
                         const float U = fmaxf(__fsub_ru(amax, x.x), __fsub_ru(x.y, amin));
@@ -293,48 +432,54 @@ __global__ void __launch_bounds__(32 * kWarps, 20) k_scan(Bufs b, int n_cand, in
                         qn += __popc(m);
                         ah = (ah + n) & (kQueue - 1);
                         an -= n;
+                        __syncwarp();
                     }
                 }
-                while (qn >= (last ? 1 : kBatch)) {
+                while (qn >= (drainall ? 1 : kBatch)) {
                     // the first queued columns against every candidate of the group
-                    __syncwarp();
                     const int n = min(qn, kBatch);
-                    float D[kBatch], x[kBatch];
+                    int col[kBatch];
+                    float d[kBatch], x[kBatch];
 #pragma unroll
                     for (int i = 0; i < kBatch; ++i) {
-                        const int col = i < n ? queue[(qh + i) & (kQueue - 1)] & ((1 << kTagShift) - 1) : 0;
-                        D[i] = __ldg(Dr + col);
-                        x[i] = __ldg(xg + (size_t)col * 32);
+                        col[i] = i < n ? queue[(qh + i) & (kQueue - 1)] : 0;
+                        d[i] = __ldg(Dr + col[i]);
+                        x[i] = __ldg(xg + (size_t)col[i] * 32);
                     }
+                    qh = (qh + n) & (kQueue - 1);
+                    qn -= n;
+                    unsigned pm = 0u;
 #pragma unroll
                     for (int i = 0; i < kBatch; ++i) {
                         const float t = __fsub_rn(xv, x[i]);
                         const float s = __fmul_rn(t, t);
-                        const float d = BWD ? __fsub_rn(D[i], s) : __fadd_rn(D[i], s);
-                        if (d <= lim && i < n) {
-                            const int e = queue[(qh + i) & (kQueue - 1)];
-                            const int tag = (int)((unsigned)e >> kTagShift);
-                            if (BWD || (tag ? tag == lane + 1 : reg)) buf[32 * nb++] = pack_key(d, e & ((1 << kTagShift) - 1));
-                        }
+                        d[i] = BWD ? __fsub_rn(d[i], s) : __fadd_rn(d[i], s);
+                        pm |= d[i] <= lim && i < n ? 1u << i : 0u;
                     }
-                    qh = (qh + n) & (kQueue - 1);
-                    qn -= n;
-                    if (__any_sync(kFull, nb > kBuf - kBatch) || (last && qn == 0 && an == 0)) {
+                    if (__any_sync(kFull, pm != 0u)) {
+#pragma unroll
+                        for (int i = 0; i < kBatch; ++i)
+                            if ((pm >> i) & 1u) buf[32 * nb++] = pack_key<BWD>(d[i], col[i]);
+                    }
+                    if (__any_sync(kFull, nb > kBuf - kBatch) || (q0 < 0 && qn == 0)) {
                         const int most = __reduce_max_sync(kFull, nb);
                         for (int j = 0; j < most; ++j) {
                             const unsigned long long key = j < nb ? buf[32 * j] : ~0ull;
                             if (key < heap[0]) sift_down(heap, K, key);
                         }
                         nb = 0;
-                        if (act) lim = key_dist(heap[0]);
+                        if (lim > -INFINITY) lim = key_dist<BWD>(heap[0]);
                         update_H();
                     }
                 }
-                if (!BWD || an < (last ? 1 : 32)) break;
+                if (!(BWD && SEED == kSeedNone) || an < (last ? 1 : 32)) break;
             }
-            if (BWD || todo == 0u) break;
-            ph = __ffs(todo) - 1;
-            todo &= todo - 1;
+        }
+        if constexpr (!BWD && SEED == kSeedHeap) {
+            if (q0 < 0 && walks) {
+                choose_walks();
+                update_H();
+            }
         }
         if (last) break;
     }
@@ -342,7 +487,7 @@ __global__ void __launch_bounds__(32 * kWarps, 20) k_scan(Bufs b, int n_cand, in
     // Epilogue: each lane's list in ascending order, padding as (FLT_MAX, 0),
     // the k-th distance for the next backward step, the optional neighbour
     // dump, labels summed in rank order.
-    if (!live) return;
+    if (!live || ((wide >> lane) & 1u)) return;
     for (int j = 0; j < nb; ++j)
         if (buf[32 * j] < heap[0]) sift_down(heap, K, buf[32 * j]);
     for (int n = K - 1; n > 0; --n) {
@@ -352,7 +497,7 @@ __global__ void __launch_bounds__(32 * kWarps, 20) k_scan(Bufs b, int n_cand, in
     }
     if (BWD) {
         const unsigned long long k = heap[(K - 1) * 32];
-        b.kth_prev[cr] = (int)(unsigned)k >= 0 ? key_dist(k) : FLT_MAX;
+        b.kth_prev[cr] = (int)(unsigned)k >= 0 ? key_dist<BWD>(k) : FLT_MAX;
     }
     if (b.nn_idx) {
         const size_t o = ((size_t)slot * b.n_rows + r) * K;
@@ -360,7 +505,7 @@ __global__ void __launch_bounds__(32 * kWarps, 20) k_scan(Bufs b, int n_cand, in
             const unsigned long long k = heap[j * 32];
             const int i = (int)(unsigned)k;
             b.nn_idx[o + j] = i >= 0 ? i : 0;
-            b.nn_dist[o + j] = i >= 0 ? key_dist(k) : FLT_MAX;
+            b.nn_dist[o + j] = i >= 0 ? key_dist<BWD>(k) : FLT_MAX;
         }
     }
     float acc = 0.0f;
@@ -412,40 +557,50 @@ __global__ void __launch_bounds__(256) k_pack_groups(Bufs b, int n_cand, int gs,
     }
 }
 
-template <bool BWD>
-cudaError_t launch_dir(const Bufs &b, int n_cand, int G, int gs, int max_smem, cudaStream_t s)
+int sm_count_scan()
 {
-    int warps = kWarps;
-    const size_t per = warp_smem(b.kmax, BWD);
-    while (warps > 1 && per * warps > (size_t)max_smem) --warps;
-    if (per * warps > (size_t)max_smem) return cudaErrorInvalidConfiguration;
-    const long long total = (long long)b.n_rows * G;
-    const long long blocks = (total + warps - 1) / warps;
-    if (total > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    auto kern = k_scan<BWD>;
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(per * warps));
-    if (e != cudaSuccess) return e;
-    // A queued column costs about 15 instructions, a sampled column stands for
-    // n / 256 of them.  A wide candidate costs n / 8 instructions and, for each
-    // of the k (1 + ln(n / k)) insertions that a list sees when columns come in
-    // random order, a heap operation with one lane at work (about 80).  Without
-    // the second term a k = 150 step of 8,192 x 4,096 took 50 ms instead of 8,
-    // the third step of a k = 50 selection from 50,021 x 24,989 86 instead of 59.
-    int wide_cost = 0;
-    if (!BWD && b.n_cols >= 4096) {
-        const double n = b.n_cols, k = b.kmax;
-        wide_cost = (int)(2.5 + 1400.0 * k * (1.0 + log(n / k > 1.0 ? n / k : 1.0)) / n);
-        if (wide_cost > 256) wide_cost = 0;
+    static const int n = [] {  // initialised once, thread-safely
+        int dev = 0, c = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev);
+        return c > 0 ? c : 148;
+    }();
+    return n;
+}
+
+template <bool BWD, int SEED, int BATCH>
+cudaError_t launch_batch(const Bufs &b, int n_cand, bool own, int max_smem, cudaStream_t s)
+{
+    const int G = scan_groups(n_cand), gs = scan_group_size(n_cand);
+    const size_t smem = warp_smem(b.kmax, BATCH, BWD || SEED == kSeedHeap);
+    const long long blocks = (long long)b.n_rows * G;
+    if (smem > (size_t)max_smem || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+    const int walks = scan_leaves_walks(b, n_cand, BWD);
+    if (walks) {
+        const cudaError_t e = cudaMemsetAsync(b.n_walk, 0, sizeof(int), s);
+        if (e != cudaSuccess) return e;
     }
-    kern<<<(unsigned)blocks, 32 * warps, per * warps, s>>>(b, n_cand, G, gs, (int)per, wide_cost);
+    auto kern = k_scan<BWD, SEED, BATCH>;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    kern<<<(unsigned)blocks, 32, smem, s>>>(b, n_cand, G, gs, walks, own ? 1 : 0);
     return cudaGetLastError();
+}
+
+template <bool BWD, int SEED>
+cudaError_t launch_seeded(const Bufs &b, int n_cand, bool own, int max_smem, cudaStream_t s)
+{
+    const long long warps = (long long)b.n_rows * scan_groups(n_cand);
+    if (warps <= (long long)sm_count_scan() * kWarpsMany) return launch_batch<BWD, SEED, kBatchFew>(b, n_cand, own, max_smem, s);
+    return launch_batch<BWD, SEED, kBatchMany>(b, n_cand, own, max_smem, s);
 }
 
 }  // namespace
 
-bool scan_supported(int n_cols, int kmax) { return n_cols < (1 << kTagShift) && kmax >= 1 && kmax <= kScoreMaxK; }
-int scan_groups(int n_cand) { return (n_cand + 31) / 32; }
-int scan_group_size(int n_cand) { return (n_cand + scan_groups(n_cand) - 1) / scan_groups(n_cand); }
+bool scan_leaves_walks(const Bufs &b, int n_cand, int backward)
+{
+    return !backward && b.sval && b.kmax <= 64 && b.n_cols >= 4096 && (long long)n_cand * b.n_rows < 0x7fffffffLL;
+}
 
 cudaError_t launch_pack_groups(const Bufs &b, int n_cand, int backward, cudaStream_t s)
 {
@@ -453,10 +608,18 @@ cudaError_t launch_pack_groups(const Bufs &b, int n_cand, int backward, cudaStre
     return cudaGetLastError();
 }
 
-cudaError_t launch_scan(const Bufs &b, int n_cand, int backward, int max_smem, cudaStream_t s)
+cudaError_t launch_scan(const Bufs &b, int n_cand, int backward, int seeding, int max_smem, cudaStream_t s)
 {
-    const int G = scan_groups(n_cand), gs = scan_group_size(n_cand);
-    return backward ? launch_dir<true>(b, n_cand, G, gs, max_smem, s) : launch_dir<false>(b, n_cand, G, gs, max_smem, s);
+    const bool own = seeding == kOwnSeeds;
+    if (backward) {
+        if (seeding == kNoSeeds) return launch_seeded<true, kSeedNone>(b, n_cand, false, max_smem, s);
+        return launch_seeded<true, kSeedHeap>(b, n_cand, true, max_smem, s);
+    }
+    // lists of up to 16: bounds from group minima; longer ones start from the seeds themselves
+    if (own || b.kmax > 16) return launch_seeded<false, kSeedHeap>(b, n_cand, own, max_smem, s);
+    if (b.kmax <= 8) return launch_seeded<false, 8>(b, n_cand, false, max_smem, s);
+    if (b.kmax <= 12) return launch_seeded<false, 12>(b, n_cand, false, max_smem, s);
+    return launch_seeded<false, 16>(b, n_cand, false, max_smem, s);
 }
 
 }  // namespace snn

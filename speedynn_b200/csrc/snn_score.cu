@@ -31,6 +31,7 @@
 #include <math.h>
 
 #include "snn_internal.h"
+#include "snn_packed.cuh"
 
 namespace snn {
 
@@ -41,31 +42,6 @@ constexpr int kCols = 32;           // columns per tile
 constexpr int kDsLd = kCols + 4;    // padded row stride of the D tile (conflict-free 128-bit reads)
 constexpr int kStages = 3;          // cp.async ring depth
 constexpr unsigned kFull = 0xffffffffu;
-
-__device__ __forceinline__ unsigned long long as_u64(float2 v) { return *reinterpret_cast<unsigned long long *>(&v); }
-__device__ __forceinline__ float2 as_f2(unsigned long long v) { return *reinterpret_cast<float2 *>(&v); }
-
-__device__ __forceinline__ float2 sub2(float2 a, float2 b)
-{
-    unsigned long long d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(as_u64(a)), "l"(as_u64(b)));
-    return as_f2(d);
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b)
-{
-    unsigned long long d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(as_u64(a)), "l"(as_u64(b)));
-    return as_f2(d);
-}
-// fl(t*t), exactly as a rounded multiply, but immune to contraction with the
-// next add (see the file comment).
-__device__ __forceinline__ float2 sq2(float2 t)
-{
-    unsigned long long d;
-    const unsigned long long z = 0ull;  // (+0.0f, +0.0f)
-    asm("fma.rn.f32x2 %0, %1, %1, %2;" : "=l"(d) : "l"(as_u64(t)), "l"(z));
-    return as_f2(d);
-}
 
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem)
 {

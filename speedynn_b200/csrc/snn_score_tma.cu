@@ -45,6 +45,7 @@
 #include <mutex>
 
 #include "snn_internal.h"
+#include "snn_packed.cuh"
 
 namespace snn {
 
@@ -68,29 +69,6 @@ constexpr unsigned long long kWaitNs = 1000000000ull;  // one second
 // Shared-memory slots per neighbour list (k <= 64).
 __host__ __device__ constexpr int list_slots(int K) { return K <= 16 ? 16 : K <= 32 ? 32 : 64; }
 
-__device__ __forceinline__ unsigned long long as_u64(float2 v) { return *reinterpret_cast<unsigned long long *>(&v); }
-__device__ __forceinline__ float2 as_f2(unsigned long long v) { return *reinterpret_cast<float2 *>(&v); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b)
-{
-    unsigned long long d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(as_u64(a)), "l"(as_u64(b)));
-    return as_f2(d);
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b)
-{
-    unsigned long long d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(as_u64(a)), "l"(as_u64(b)));
-    return as_f2(d);
-}
-// fl(t*t) via fma(t, t, +0): a packed mul.rn feeding an add.rn is contracted
-// into one FMA by ptxas; the fma form keeps the reference's two roundings.
-__device__ __forceinline__ float2 sq2(float2 t)
-{
-    unsigned long long d;
-    const unsigned long long z = 0ull;
-    asm("fma.rn.f32x2 %0, %1, %1, %2;" : "=l"(d) : "l"(as_u64(t)), "l"(z));
-    return as_f2(d);
-}
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
 {
     unsigned long long d;
@@ -472,7 +450,7 @@ __global__ void __launch_bounds__(256) k_seed_bounds_exact(Bufs b, int n_cand, i
 // distances count as +inf.  One warp per row, lane l holding seeds
 // l + 32 j (j < kSeedsPerLane); the gathers of two candidates are issued
 // together, and many warps per SM hide their latency.  Each lane keeps its
-// V smallest values (V = 4 up to K = 128, all 8 above), and the K-th smallest of
+// V = 4 smallest values, and the K-th smallest of
 // those 32 V values is the bound: a subset of the seeds, so still K distinct
 // columns, and as tight as all of them unless a lane holds more than V of
 // the K nearest.
@@ -1074,8 +1052,7 @@ cudaError_t launch_seed_bounds(const Bufs &b, int n_cand, cudaStream_t s)
     else if (b.kmax <= 8) k_seed_bounds_exact<8><<<grid, 256, 0, s>>>(b, n_cand, G, gs, b.bound);
     else if (b.kmax <= 12) k_seed_bounds_exact<12><<<grid, 256, 0, s>>>(b, n_cand, G, gs, b.bound);
     else if (b.kmax <= 16) k_seed_bounds_exact<16><<<grid, 256, 0, s>>>(b, n_cand, G, gs, b.bound);
-    else if (b.kmax <= 128) k_seed_bounds<4><<<grid, 256, 0, s>>>(b, n_cand, b.bound);
-    else k_seed_bounds<8><<<grid, 256, 0, s>>>(b, n_cand, b.bound);
+    else k_seed_bounds<4><<<grid, 256, 0, s>>>(b, n_cand, b.bound);
     return cudaGetLastError();
 }
 

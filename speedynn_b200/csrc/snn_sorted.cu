@@ -365,77 +365,71 @@ __device__ __forceinline__ void warp_sort64x2(unsigned long long (&v)[2], int la
     }
 }
 
-// k_second_step_long: the walk of k_second_step for 32 < k <= 64.  The list
-// sits as adjacent pairs (lane j holds entries 2j and 2j+1), so an insertion
-// shifts it with one shuffle per array; and the first 64 columns (32 per side,
-// or 64 on the side still open) are read together and sorted into the list at
-// once, so with k finite distances among them the list is full -- and the
-// walk's sides can finish -- from the first batch on.
-__global__ void __launch_bounds__(256, 8) k_second_step_long(Bufs b, const float *sv, const int *si, const float *xs,
-                                                          int n_cand, unsigned long long *walked,
-                                                          unsigned long long budget)
+// The k (<= 64) nearest columns of scored row r for candidate slot `slot` by an
+// outward walk of one feature's n sorted training values bv (columns bi) from
+// a: the distance is fl(f + g) >= f with f = fl((a - bv)^2), so a side is
+// finished once its next f exceeds the k-th distance.  pre(j, in) loads what g
+// needs for sorted position j, dist(f, pre, i) forms the distance of column i.
+// th: an inclusive bound on the k-th distance, or +inf.  stop() is asked every
+// 64 iterations of 32 U columns.  The list sits as adjacent pairs (lane j holds entries 2j and
+// 2j+1), ordered by (distance, index) since columns arrive out of index order,
+// so an insertion shifts it with one shuffle per array; the first 64 columns
+// (32 per side, or 64 on the side still open) are read together and sorted into
+// the list at once, so with k distances below the bound among them the list is
+// full -- and the walk's sides can finish -- from the first batch on.
+// Returns false if stop() ended the walk; else the list is written out.
+template <int U, class Pre, class Dist, class Stop>
+__device__ __forceinline__ bool walk_lists(const Bufs &b, int r, int slot, float a, bool finite, const float *bv, const int *bi,
+                                           float th, Pre pre, Dist dist, Stop stop)
 {
     constexpr unsigned kFull = 0xffffffffu;
-    if (b.st->done) return;
     const int lane = threadIdx.x & 31;
-    const int slot = blockIdx.y;
-    const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (slot >= n_cand || r >= b.n_rows) return;  // warp-uniform
     const int K = b.kmax;
     const int n = b.n_cols;
-    const int w = b.st->winner;
-    const int c = b.cands[slot];
-    const float aw = b.XV[(size_t)w * b.ldr + r];
-    const float ac = b.XV[(size_t)c * b.ldr + r];
-    const float *bv = sv + (size_t)w * b.ldc;
-    const int *bi = si + (size_t)w * b.ldc;
-    const float *xsc = xs + (size_t)slot * b.ldc;
     // the list: entries e0 = 2 * lane and e0 + 1 (valid below cnt)
     const int e0 = 2 * lane;
     float2 Lv = make_float2(INFINITY, INFINITY);
     int2 Iv = make_int2(0x7fffffff, 0x7fffffff);
     int cnt = 0;
-    float th = INFINITY;  // the k-th entry once the list is full
-    int thi = 0x7fffffff;
-    // non-finite x_r,w or x_r,c: no distance below FLT_MAX, the list stays padding
-    if (isfinite(aw) && isfinite(ac)) {
+    int thi = 0x7fffffff;  // th and thi: the k-th entry once the list is full
+    if (finite) {  // otherwise no distance is below FLT_MAX: the list stays padding
         int lo = 0, hi = n;
         while (lo < hi) {
             const int mid = (lo + hi) >> 1;
-            if (bv[mid] < aw) lo = mid + 1;
+            if (bv[mid] < a) lo = mid + 1;
             else hi = mid;
         }
         int ln = lo - 1, rn = lo;  // next unvisited position on each side
         bool ldone = ln < 0, rdone = rn >= n;
         // batch position q: the left side's (q+1)-th next column for q < nl, else the right side's
-        auto visit = [&](int q, int nl, float &D, float &d, int &i) {
+        auto visit = [&](int q, int nl, float &f, float &d, int &i) {
             const bool left = q < nl;
             const int j = left ? ln - q : rn + (q - nl);
             const bool in = left ? j >= 0 : (!rdone && j < n);
-            // the three loads are independent (and contiguous across the lanes)
-            const float vj = in ? bv[j] : 0.0f, xj = in ? xsc[j] : 0.0f;
+            // independent loads, contiguous across the lanes
+            const float vj = in ? bv[j] : 0.0f, gj = pre(j, in);
             const int ij = in ? bi[j] : 0x7fffffff;
-            D = in ? dist1(aw, vj) : INFINITY;
+            f = in ? dist1(a, vj) : INFINITY;
             d = INFINITY;
             i = 0x7fffffff;
-            if (in && D <= th) {  // d >= D: beyond the k-th distance nothing enters
+            if (in && f <= th) {  // d >= f: beyond the k-th distance nothing enters
                 i = ij;
-                const float t = __fsub_rn(ac, xj);
-                d = __fadd_rn(D, __fmul_rn(t, t));
+                d = dist(f, gj, ij);
             }
         };
         if (!(ldone && rdone)) {
-            // first batch, 64 columns: their finite distances sorted by (distance, index)
-            // (distances are >= +0, so their bits order like the values), the first K kept
+            // first batch, 64 columns: their distances within the bound sorted by
+            // (distance, index) (distances are >= +0, so their bits order like the
+            // values), the first K kept
             const int nl = ldone ? 0 : (rdone ? 64 : 32);
-            float Da, da, Db, db;
+            float fa, da, fb, db;
             int ia, ib;
-            visit(lane, nl, Da, da, ia);
-            visit(lane + 32, nl, Db, db, ib);
-            unsigned long long kk[2] = {
-                da < FLT_MAX ? ((unsigned long long)__float_as_uint(da) << 32) | (unsigned)ia : ~0ull,
-                db < FLT_MAX ? ((unsigned long long)__float_as_uint(db) << 32) | (unsigned)ib : ~0ull};
-            cnt = min(__popc(__ballot_sync(kFull, da < FLT_MAX)) + __popc(__ballot_sync(kFull, db < FLT_MAX)), K);
+            visit(lane, nl, fa, da, ia);
+            visit(lane + 32, nl, fb, db, ib);
+            const bool ka = da < FLT_MAX && da <= th, kb = db < FLT_MAX && db <= th;
+            unsigned long long kk[2] = {ka ? ((unsigned long long)__float_as_uint(da) << 32) | (unsigned)ia : ~0ull,
+                                        kb ? ((unsigned long long)__float_as_uint(db) << 32) | (unsigned)ib : ~0ull};
+            cnt = min(__popc(__ballot_sync(kFull, ka)) + __popc(__ballot_sync(kFull, kb)), K);
             warp_sort64x2(kk, lane);
             if (e0 < cnt) {
                 Lv.x = __uint_as_float((unsigned)(kk[0] >> 32));
@@ -449,69 +443,71 @@ __global__ void __launch_bounds__(256, 8) k_second_step_long(Bufs b, const float
                 th = __shfl_sync(kFull, ((K - 1) & 1) ? Lv.y : Lv.x, (K - 1) >> 1);
                 thi = __shfl_sync(kFull, ((K - 1) & 1) ? Iv.y : Iv.x, (K - 1) >> 1);
             }
-            // a side is finished past its end or once its farthest D of the batch exceeds the k-th
+            // a side is finished past its end or once its farthest f of the batch exceeds the k-th
             const int ql = nl > 0 ? nl - 1 : 0;
-            const float dl_far = __shfl_sync(kFull, ql < 32 ? Da : Db, ql & 31);
-            const float dr_far = __shfl_sync(kFull, Db, 31);
+            const float fl_far = __shfl_sync(kFull, ql < 32 ? fa : fb, ql & 31);
+            const float fr_far = __shfl_sync(kFull, fb, 31);
             ln -= nl;
             rn += 64 - nl;
-            ldone = ldone || ln < 0 || (nl > 0 && dl_far > th);
-            rdone = rdone || rn >= n || (nl < 64 && dr_far > th);
+            ldone = ldone || ln < 0 || (nl > 0 && fl_far > th);
+            rdone = rdone || rn >= n || (nl < 64 && fr_far > th);
         }
         for (int it = 1; !(ldone && rdone); ++it) {
-            if ((it & 63) == 0) {  // account for the walk; leave when the budget is spent
-                int stop = 0;
-                if (lane == 0) {
-                    const unsigned long long tot = atomicAdd(walked, 64ull * 32ull) + 64ull * 32ull;
-                    if (tot > budget) atomicExch(&b.st->full_scan, 1);
-                    stop = tot > budget || *(volatile int *)&b.st->full_scan;
-                }
-                if (__shfl_sync(kFull, stop, 0)) return;
-            }
-            // 16 columns per side, or all 32 lanes on the side still open
-            const int nl = ldone ? 0 : (rdone ? 32 : 16);
-            float D, d;
-            int i;
-            visit(lane, nl, D, d, i);
-            unsigned m = __ballot_sync(kFull, d < FLT_MAX && (d < th || (d == th && i < thi)));
-            while (m) {
-                const int l = __ffs(m) - 1;
-                m &= m - 1;
-                const float dv = __shfl_sync(kFull, d, l);
-                const int iv = __shfl_sync(kFull, i, l);
-                if (!(dv < th || (dv == th && iv < thi))) continue;  // the list tightened meanwhile
-                // position: entries ordered before (dv, iv)
-                const int pos = __popc(__ballot_sync(kFull, e0 < cnt && (Lv.x < dv || (Lv.x == dv && Iv.x < iv)))) +
-                                __popc(__ballot_sync(kFull, e0 + 1 < cnt && (Lv.y < dv || (Lv.y == dv && Iv.y < iv))));
-                const float pL = __shfl_up_sync(kFull, Lv.y, 1);  // entry 2j - 1
-                const int pI = __shfl_up_sync(kFull, Iv.y, 1);
-                // entry 2j + 1 first: it may take the old entry 2j
-                if (e0 + 1 == pos) {
-                    Lv.y = dv;
-                    Iv.y = iv;
-                } else if (e0 + 1 > pos && e0 + 1 < K) {
-                    Lv.y = Lv.x;
-                    Iv.y = Iv.x;
-                }
-                if (e0 == pos) {
-                    Lv.x = dv;
-                    Iv.x = iv;
-                } else if (e0 > pos && e0 < K) {
-                    Lv.x = pL;
-                    Iv.x = pI;
-                }
-                if (cnt < K) ++cnt;
-                if (cnt == K) {
-                    th = __shfl_sync(kFull, ((K - 1) & 1) ? Lv.y : Lv.x, (K - 1) >> 1);
-                    thi = __shfl_sync(kFull, ((K - 1) & 1) ? Iv.y : Iv.x, (K - 1) >> 1);
+            if ((it & 63) == 0 && stop()) return false;
+            // 16 U columns per side, or 32 U on the side still open, U per lane
+            const int nl = ldone ? 0 : (rdone ? 32 * U : 16 * U);
+            float f[U], d[U];
+            int i[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) visit(32 * u + lane, nl, f[u], d[u], i[u]);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                unsigned m = __ballot_sync(kFull, d[u] < FLT_MAX && (d[u] < th || (d[u] == th && i[u] < thi)));
+                while (m) {
+                    const int l = __ffs(m) - 1;
+                    m &= m - 1;
+                    const float dv = __shfl_sync(kFull, d[u], l);
+                    const int iv = __shfl_sync(kFull, i[u], l);
+                    if (!(dv < th || (dv == th && iv < thi))) continue;  // the list tightened meanwhile
+                    // position: entries ordered before (dv, iv)
+                    const int pos = __popc(__ballot_sync(kFull, e0 < cnt && (Lv.x < dv || (Lv.x == dv && Iv.x < iv)))) +
+                                    __popc(__ballot_sync(kFull, e0 + 1 < cnt && (Lv.y < dv || (Lv.y == dv && Iv.y < iv))));
+                    const float pL = __shfl_up_sync(kFull, Lv.y, 1);  // entry 2j - 1
+                    const int pI = __shfl_up_sync(kFull, Iv.y, 1);
+                    // entry 2j + 1 first: it may take the old entry 2j
+                    if (e0 + 1 == pos) {
+                        Lv.y = dv;
+                        Iv.y = iv;
+                    } else if (e0 + 1 > pos && e0 + 1 < K) {
+                        Lv.y = Lv.x;
+                        Iv.y = Iv.x;
+                    }
+                    if (e0 == pos) {
+                        Lv.x = dv;
+                        Iv.x = iv;
+                    } else if (e0 > pos && e0 < K) {
+                        Lv.x = pL;
+                        Iv.x = pI;
+                    }
+                    if (cnt < K) ++cnt;
+                    if (cnt == K) {
+                        th = __shfl_sync(kFull, ((K - 1) & 1) ? Lv.y : Lv.x, (K - 1) >> 1);
+                        thi = __shfl_sync(kFull, ((K - 1) & 1) ? Iv.y : Iv.x, (K - 1) >> 1);
+                    }
                 }
             }
-            // a side is finished past its end or once its farthest D of this batch exceeds the k-th
-            const float dl_far = __shfl_sync(kFull, D, nl > 0 ? nl - 1 : 0), dr_far = __shfl_sync(kFull, D, 31);
+            // a side is finished past its end or once its farthest f of this batch exceeds the k-th
+            float fl_far = 0.0f;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const float v = __shfl_sync(kFull, f[u], (nl - 1) & 31);
+                if (u == (nl - 1) >> 5) fl_far = v;
+            }
+            const float fr_far = __shfl_sync(kFull, f[U - 1], 31);
             ln -= nl;
-            rn += 32 - nl;
-            ldone = ldone || ln < 0 || (nl > 0 && dl_far > th);
-            rdone = rdone || rn >= n || (nl < 32 && dr_far > th);
+            rn += 32 * U - nl;
+            ldone = ldone || ln < 0 || (nl > 0 && fl_far > th);
+            rdone = rdone || rn >= n || (nl < 32 * U && fr_far > th);
         }
     }
     // entries past cnt are padding (FLT_MAX, 0)
@@ -546,6 +542,63 @@ __global__ void __launch_bounds__(256, 8) k_second_step_long(Bufs b, const float
                 const int k = __ldg(b.kvals + m);
                 if (k == e + 1) b.pred[((size_t)slot * b.nk + m) * b.n_rows + r] = __fdiv_rn(acc, (float)k);
             }
+    }
+    return true;
+}
+
+// k_second_step_long: the walk of k_second_step for 32 < k <= 64.
+__global__ void __launch_bounds__(256, 8) k_second_step_long(Bufs b, const float *sv, const int *si, const float *xs,
+                                                          int n_cand, unsigned long long *walked,
+                                                          unsigned long long budget)
+{
+    if (b.st->done) return;
+    const int lane = threadIdx.x & 31;
+    const int slot = blockIdx.y;
+    const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (slot >= n_cand || r >= b.n_rows) return;  // warp-uniform
+    const int w = b.st->winner;
+    const int c = b.cands[slot];
+    const float aw = b.XV[(size_t)w * b.ldr + r];
+    const float ac = b.XV[(size_t)c * b.ldr + r];
+    const float *xsc = xs + (size_t)slot * b.ldc;
+    walk_lists<1>(
+        b, r, slot, aw, isfinite(aw) && isfinite(ac), sv + (size_t)w * b.ldc, si + (size_t)w * b.ldc, INFINITY,
+        [&](int j, bool in) { return in ? xsc[j] : 0.0f; },
+        [&](float f, float x, int) {
+            const float t = __fsub_rn(ac, x);
+            return __fadd_rn(f, __fmul_rn(t, t));
+        },
+        [&] {  // account for the walk; leave when the budget is spent
+            int stop = 0;
+            if (lane == 0) {
+                const unsigned long long tot = atomicAdd(walked, 64ull * 32ull) + 64ull * 32ull;
+                if (tot > budget) atomicExch(&b.st->full_scan, 1);
+                stop = tot > budget || *(volatile int *)&b.st->full_scan;
+            }
+            return __shfl_sync(0xffffffffu, stop, 0) != 0;
+        });
+}
+
+// k_walk: the (candidate, row) problems that the pruned scan left out because
+// the row is an outlier in the candidate's feature (snn_scan.cu).  There the
+// candidate's own square decides who is near: the walk goes outwards in the
+// candidate's sorted values and gathers D.  On the fwd-64k data such a walk
+// visits 4 % of the columns, while 15 to 35 % have D within the problem's bound.
+// One warp per problem, taken in turn; b.bound holds the problems' bounds.  The
+// gathers of D bound it (one memory sector per column), so each lane has four
+// in flight.
+__global__ void __launch_bounds__(256, 4) k_walk(Bufs b)
+{
+    if (b.st->done) return;
+    const int total = *b.n_walk;
+    for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < total; i += gridDim.x * (blockDim.x >> 5)) {
+        const int slot = b.walk[i] / b.n_rows, r = b.walk[i] % b.n_rows;
+        const int c = b.cands[slot];
+        const float *Dr = b.D + (size_t)r * b.ldc;
+        walk_lists<4>(
+            b, r, slot, b.XV[(size_t)c * b.ldr + r], true, b.sval + (size_t)c * b.ldc, b.sidx + (size_t)c * b.ldc,
+            b.bound[(size_t)c * b.n_rows + r], [](int, bool) { return 0.0f; },
+            [&](float f, float, int i) { return __fadd_rn(__ldg(Dr + i), f); }, [] { return false; });
     }
 }
 
@@ -584,6 +637,19 @@ cudaError_t launch_second_step(const Bufs &b, const float *sv, const int *si, fl
     if (b.kmax <= 32) k_second_step<<<grid, 256, 0, s>>>(b, sv, si, xs, n_cand, walked, budget);
     else if (b.kmax <= 64) k_second_step_long<<<grid, 256, 0, s>>>(b, sv, si, xs, n_cand, walked, budget);
     else return cudaErrorInvalidValue;  // k above 64 scans
+    return cudaGetLastError();
+}
+
+cudaError_t launch_walk(const Bufs &b, cudaStream_t s)
+{
+    if (b.kmax > 64) return cudaErrorInvalidValue;
+    static const int sms = [] {  // initialised once, thread-safely
+        int dev = 0, c = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev);
+        return c > 0 ? c : 148;
+    }();
+    k_walk<<<sms * 4, 256, 0, s>>>(b);
     return cudaGetLastError();
 }
 
