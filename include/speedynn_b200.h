@@ -211,16 +211,18 @@ SNN_API int snn_get_timing(snn_handle *h, double *score_ms, int *score_launches,
  *                  by the previous commit) instead of a first pass over a
  *                  quarter of the columns; steps with such bounds are scored
  *                  by the pruned scan.  Results are identical; only the work
- *                  differs.  Default 2 for a holdout problem with k_max <= 64
- *                  (its first two steps run from sorted columns), else 1; a
+ *                  differs.  Default: the first step that does not run from
+ *                  sorted columns (SNN_OPT_SORTED_START) and has a commit
+ *                  behind it; with kernel 3 step 2 (3 when k_max > 16).  A
  *                  large value turns it off. */
 #define SNN_OPT_SEED_STEP 4
 /*   SNN_OPT_SORTED_START 1 (default): the first two forward steps of a
- *                  holdout problem take their lists from training values
- *                  sorted at load instead of a scan.  Step 1 (nothing
- *                  committed, every candidate's distances one-dimensional): a
- *                  binary search and a short outward walk per (row,
- *                  candidate).  Step 2 (one feature committed): a walk of that
+ *                  holdout problem may take their lists from training values
+ *                  sorted at load.  Step 1 (nothing committed, every
+ *                  candidate's distances one-dimensional): a binary search and
+ *                  a short outward walk per (row, candidate).  Step 2 (one
+ *                  feature committed; with the automatic kernel choice only
+ *                  up to 4,096 training rows and k_max <= 32): a walk of that
  *                  feature's sorted values in increasing committed distance,
  *                  ended once it exceeds the candidate's k-th distance.  Data
  *                  with too many tied distances fall back to the scan.  0:

@@ -109,7 +109,7 @@ struct snn_handle {
     int *walk = nullptr, *n_walk = nullptr;  // forward holdout: problems left to k_walk, and how many
     bool sorted_start = true;     // SNN_OPT_SORTED_START
     bool seeds_ok = false;        // seeds hold the current D's seed columns
-    int seed_step = 2;            // SNN_OPT_SEED_STEP: first forward step scored from seed bounds (set at create)
+    int seed_step = 0;            // SNN_OPT_SEED_STEP: first forward step scored from seed bounds; 0: first_seeded
     unsigned long long *fcount = nullptr;  // filter counters of the TMA-fed scorer (3)
     bool count_filter = false;             // SNN_OPT_COUNTERS
     int kernel = 0;               // scoring kernel: 0 auto, 1 rows per lane, 3 TMA-fed row tiles
@@ -289,17 +289,39 @@ int check_device(int device)
 // the rows-per-lane scorer (any k_max <= 256).
 bool use_tma(const snn_handle *h) { return h->kernel == 3 || (h->kernel == 0 && snn::score_tma_supported(h->kmax)); }
 
-// Forward step t (t features committed) is scored from seed bounds once
-// t >= seed_step: the columns nearest under D are mostly near under D + one
-// more feature too, so any k of 256 of them bound the k-th distance well.  The
-// sorted columns of a holdout problem score its first two steps (k <= 64)
-// faster; everything else starts with the first step that has a commit behind
-// it (step 1 of a 3000-row CV problem: 0.23 ms by the scan from seed bounds,
-// 0.57 ms dense with a first pass; step 2 of fwd-64k: 9.9 against 31 ms).  The
-// commit before such a step writes the seeds.
+// The first two forward steps of a holdout problem can run from sorted feature
+// columns (D is zero, then one-dimensional there); CV mode excludes same-fold
+// pairs.  The second step walks one warp per problem, which the automatic
+// choice takes only where the problem is small (2,000 x 1,000 x 20: 0.09 ms,
+// the scan 0.11; 5,003 x 2,501 x 24, k = 15: 0.32 against 0.26; fwd-64k 13.7
+// against 10.2; 50,021 x 24,989 x 100, k = 50: 60 against 44).
+constexpr int kSortedSecondCols = 4096;
+bool sorted_step(const snn_handle *h, int t)
+{
+    if (!h->sorted_start || !h->sval || h->desc.backward || h->cv) return false;
+    if (t == 0) return true;
+    if (t != 1 || h->kmax > 64) return false;  // the second step's walk keeps at most 64 entries
+    return h->kernel != 0 || (h->kmax <= 32 && h->n_cols <= kSortedSecondCols);
+}
+
+// First forward step scored from seed bounds: the columns nearest under D are
+// mostly near under D + one more feature too, so any k of 256 of them bound
+// the k-th distance well.  The scan takes every step with a commit behind it
+// and no sorted columns (step 1 of a 3000-row CV problem: 0.17 ms, 0.57 dense
+// with a first pass; step 2 of fwd-64k 6.2 against 31).  For the dense
+// scorers one committed feature is too few (fwd-64k: 21 % of rows flagged with
+// a first pass, 18 % seeded at step 2, not below it at step 1), with k above 16
+// two are (fwd-200k step 2: 845 ms, 913 seeded).  The commit before such a step
+// writes the seeds.
+int first_seeded(const snn_handle *h)
+{
+    if (h->seed_step) return h->seed_step;
+    if (h->kernel == 0) return sorted_step(h, 1) ? 2 : 1;
+    return h->kmax <= 16 ? 2 : 3;
+}
 bool seeds_for_step(const snn_handle *h, int t)
 {
-    return !h->desc.backward && h->seeds && h->kernel != 1 && t >= h->seed_step;
+    return !h->desc.backward && h->seeds && h->kernel != 1 && t >= first_seeded(h);
 }
 
 // How the automatic choice scores step t by the pruned scan (snn_scan.cu): the
@@ -318,15 +340,6 @@ int scan_seeding(const snn_handle *h, int t, bool seeded)
     if (h->desc.backward) return h->prev_ok ? snn::kNoSeeds : snn::kOwnSeeds;
     if (seeded) return snn::kGivenSeeds;
     return t == 0 && h->n_cols <= kScanAllCols ? snn::kOwnSeeds : -1;
-}
-
-// The first two forward steps of a holdout problem run from sorted feature
-// columns (D is zero, then one-dimensional there); CV mode excludes same-fold
-// pairs and takes the scan.
-bool sorted_step(const snn_handle *h, int t)
-{
-    if (!h->sorted_start || !h->sval || h->desc.backward || h->cv) return false;
-    return t == 0 || (t == 1 && h->kmax <= 64);  // the second step's walk keeps at most 64 entries
 }
 
 // Issue one greedy step (no synchronisation).
@@ -603,7 +616,6 @@ SNN_API int snn_create(const snn_desc *d, snn_handle **out)
     h->n_rows = cv ? d->n_train : d->n_val;
     h->npf = cv ? d->n_train / d->k_fold : 1;
     h->kmax = kmax;
-    h->seed_step = cv || kmax > 64 ? 1 : 2;
     h->nk = d->num_k_vals;
     h->ldc = round_up(h->n_cols, snn::kPadCols);
     h->ldr = cv ? h->ldc : round_up(h->n_rows, snn::kPadCols);

@@ -26,8 +26,13 @@
 //     128-byte line per column and group, so a gather is one full-width load);
 //     every lane forms its candidate's exact distance and appends it to its
 //     own buffer in shared memory if it may enter the list;
+//   * forward, where the bounds still reach beyond the row's 1,024 nearest columns
+//     (under the committed D), these are taken first: they leave nearly exact
+//     bounds, and the second pass over the row finds little open (k = 50, third
+//     step of 50,021 x 24,989: 38 -> 30 ms) or is not needed;
 //   * when a lane's buffer is half full, all lanes empty theirs together into
-//     their lists, heaps of k_max (distance, column) keys in shared memory.  The
+//     their lists, heaps of k_max (distance, column) keys in shared memory (four
+//     children per node: k = 50 selection 335 -> 314 ms against two).  The
 //     keys are ordered by distance, then column, which is the reference's
 //     stable rule in whatever order the columns arrive;
 //   * forward, a row that is an outlier in a feature leaves that candidate's
@@ -42,11 +47,11 @@
 //
 // What bounds it: instruction issue (55 to 60 % of the slots; the rest is each
 // warp's own chain) well above the D stream: fwd-64k 3.3 ms per late step, 1.3 ms
-// of it the read of D.  Scoring of a whole fwd-64k selection 293 -> 71 ms
+// of it the read of D.  Scoring of a whole fwd-64k selection 293 -> 66 ms
 // (80 with the bounds in a kernel of their own and the outliers scanned here
 // with lane = column, 128 columns per exposed load), a backward step of 25,003
-// x 12,502 7.0 -> 1.0 ms, a k = 50 step of 50,021 x 24,989 57 -> 13 ms, a
-// k = 150 step of 8,192 x 4,096 x 19 130 -> 6 ms.
+// x 12,502 7.0 -> 1.0 ms, a k = 50 step of 50,021 x 24,989 57 -> 12 ms, a
+// k = 150 step of 8,192 x 4,096 x 19 130 -> 4 ms.
 #include <float.h>
 #include <math.h>
 #include <stdint.h>
@@ -64,9 +69,10 @@ constexpr int kCols = 128 * kUnroll;  // columns per pass of the loop
 constexpr int kQueue = 256;           // entries of a warp's column queues (a power of two, kSeeds at least)
 constexpr float kCap = 0x1.fffffcp+127f;  // largest distance that can enter a list (items at FLT_MAX never do)
 // Instructions of a warp, for choosing who walks (k_scan): a queued column, the
-// start of a walk, a column of it (1.6 instructions, but its gather of D fetches
+// start of a walk, a column of it, a column of another pass over the row (a walk's column: 1.6 instructions, but its gather of D fetches
 // 64 bytes from memory, worth more; fwd-64k 120 ms a selection at 4, 118 at 9).
-constexpr float kQueueCost = 14.0f, kWalkStart = 3000.0f, kWalkCost = 8.0f;
+constexpr float kQueueCost = 14.0f, kWalkStart = 3000.0f, kWalkCost = 8.0f, kPassCost = 0.2f;
+constexpr int kNear = 1024;  // columns of a row taken first (a power of two times kSeeds)
 static_assert(kQueue >= kSeeds && kQueue >= 128 + 16 + 32, "room for a pass's columns");
 
 // Order-preserving signed key of a float (no NaN), and back.
@@ -93,24 +99,22 @@ __device__ __forceinline__ float key_dist(unsigned long long k)
     return BWD ? fkey_inv((int)(u ^ 0x80000000u)) : __uint_as_float(u);
 }
 
-// Replace the root of the lane's max-heap h[0], h[32], ... (n entries) by key.
-__device__ __forceinline__ void sift_down(unsigned long long *h, int n, unsigned long long key)
+// Put key in the place of entry i of the lane's max-heap h[0], h[32], ... (n
+// entries, four children per node: half the dependent levels of a binary heap)
+// and sink it.
+__device__ __forceinline__ void sift_down(unsigned long long *h, int n, unsigned long long key, int i = 0)
 {
-    int i = 0;
-    for (;;) {
-        int l = 2 * i + 1;
-        if (l >= n) break;
-        unsigned long long kl = h[l * 32];
-        if (l + 1 < n) {
-            const unsigned long long kr = h[(l + 1) * 32];
-            if (kr > kl) {
-                kl = kr;
-                ++l;
-            }
-        }
-        if (key >= kl) break;
-        h[i * 32] = kl;
-        i = l;
+    for (int c = 4 * i + 1; c < n; c = 4 * i + 1) {
+        const unsigned long long *p = h + c * 32;
+        const unsigned long long k0 = p[0], k1 = c + 1 < n ? p[32] : 0ull, k2 = c + 2 < n ? p[64] : 0ull,
+                                 k3 = c + 3 < n ? p[96] : 0ull;
+        const bool a = k1 > k0, d = k3 > k2;
+        const unsigned long long ka = a ? k1 : k0, kd = d ? k3 : k2;
+        const bool e = kd > ka;
+        const unsigned long long k = e ? kd : ka;
+        if (key >= k) break;
+        h[i * 32] = k;
+        i = c + (e ? (d ? 3 : 2) : (a ? 1 : 0));
     }
     h[i * 32] = key;
 }
@@ -164,6 +168,21 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
     const float4 *row = reinterpret_cast<const float4 *>(Dr);
     const int n4 = b.ldc >> 2;
 
+    // near: about the kNear-th smallest committed distance of the row, from the
+    // lanes' 4th and 8th nearest seeds (about the 128th and 256th of the row),
+    // continued as the power law that runs through their means.
+    float near = INFINITY;
+    auto set_near = [&](float d4, float d8) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            d4 += __shfl_xor_sync(kFull, d4, o);
+            d8 += __shfl_xor_sync(kFull, d8, o);
+        }
+        float v = d8 * 0.03125f;
+        for (int m = kSeeds; m < kNear; m *= 2) v *= d8 / d4;
+        if (v < FLT_MAX) near = v;  // otherwise (a lane without eight seeds, ties at 0): one stage for all columns
+    };
+
     // lim: distances above it cannot enter the lane's list.
     float lim = act ? kCap : -INFINITY;
     if (BWD && SEED == kSeedNone && act) lim = fminf(b.kth_prev[cr], kCap);
@@ -214,20 +233,34 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
             }
         }
         if (act) lim = fminf(L[SEED - 1], kCap);
+        set_near(__ldg(seed_d + 3 * 32), __ldg(seed_d + 7 * 32));
     }
 
     // The list starts as K sentinels at the (inclusive) bound, ordered after every
     // column; those left at the end are padding.
+    // They give way from the last entry up, where a key sinks through few levels
+    // or none; once all are gone (put is 0), a key replaces the largest entry.
     for (int j = 0; j < K; ++j) heap[j * 32] = pack_key<BWD>(lim, -1);
+    // (Not beside the second test, whose registers are all in use.)
+    int put = BWD && SEED == kSeedNone ? 0 : K - 1;
+    auto enter = [&](unsigned long long key) {
+        if (key < heap[put * 32]) {
+            sift_down(heap, K, key, put);
+            if (!(BWD && SEED == kSeedNone)) put = max(put - 1, 0);
+        }
+    };
 
     int qh = 0, qn = 0;  // queue: first entry, entries
     // kSeedHeap: the seed columns go through the queue before the row's others; the
     // lane keeps its own (the commit and this kernel give each lane the same
     // columns), ascending, to leave them out afterwards.
-    int nseed = 0;  // the lane's seed columns not yet passed, the last ones at aux[32 * i + lane]
+    int nseed = 0;  // the lane's seed columns already passed, the next at aux[32 * nseed + lane]
+    int noseed = 0;  // entries of aux without a column
     if constexpr (SEED == kSeedHeap) {
         int si[kSeedsPerLane];
         if (!own) {
+            const float *seed_d = b.seed_d + (size_t)r * kSeeds + lane;
+            if (!BWD) set_near(__ldg(seed_d + 3 * 32), __ldg(seed_d + 7 * 32));
 #pragma unroll
             for (int j = 0; j < kSeedsPerLane; ++j) si[j] = __ldg(b.seeds + (size_t)r * kSeeds + j * 32 + lane);
         } else {
@@ -259,14 +292,16 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
                     }
                 }
             }
+            if (!BWD) set_near(sv[3], sv[7]);
         }
 #pragma unroll
         for (int j = 0; j < kSeedsPerLane; ++j) {  // nearest first
             const unsigned m = __ballot_sync(kFull, si[j] >= 0);
             if (si[j] >= 0) queue[qn + __popc(m & ((1u << lane) - 1u))] = si[j];
             qn += __popc(m);
-            nseed += si[j] >= 0 ? 1 : 0;
+            noseed += si[j] >= 0 ? 0 : 1;
         }
+        nseed = noseed;
 #pragma unroll
         for (int i = 1; i < kSeedsPerLane; ++i)  // ascending, absent ones (-1) first
 #pragma unroll
@@ -331,7 +366,8 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
         }
         const float n = (float)b.n_cols;
         const int walk = (int)(kWalkStart + kWalkCost / 64.0f * n * (float)cs);
-        int cost = (int)(kQueueCost / 128.0f * n * (float)cd);  // if the candidates with more columns walk
+        // if the candidates with more columns walk; beyond near the row is read once more
+        int cost = (int)(kQueueCost / 128.0f * n * (float)cd + (lim >= near ? kPassCost * n : 0.0f));
 #pragma unroll 4
         for (int l = 0; l < 32; ++l) {
             const int wl = __shfl_sync(kFull, walk, l), cl = __shfl_sync(kFull, cd, l);
@@ -354,29 +390,55 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
 
     int nb = 0;  // the lane's buffered keys
     int ah = 0, an = 0;  // backward: columns that wait for the second test (aux)
-    constexpr int q_first = SEED == kSeedHeap ? -kCols : 0;  // a pass for the seed columns first
-    if constexpr (!BWD && SEED != kSeedHeap) {
-        if (walks) choose_walks();
-    }
+    auto flush = [&] {
+        const int most = __reduce_max_sync(kFull, nb);
+        for (int j = 0; j < most; ++j) {
+            const unsigned long long key = j < nb ? buf[32 * j] : ~0ull;
+            enter(key);
+        }
+        nb = 0;
+        if (lim > -INFINITY) lim = key_dist<BWD>(heap[0]);
+        update_H();
+    };
     update_H();
-    float4 nxt[kUnroll];
-#pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-        const int q = u * 32 + lane;
-        nxt[u] = q < n4 ? __ldg(row + q) : make_float4(INFINITY, INFINITY, INFINITY, INFINITY);
+    // Forward, two stages where the bounds still reach beyond near: its columns
+    // first, which leaves nearly exact bounds for the split and for the others
+    // (or none of them open).
+    int stage = BWD || !(H > near) ? 2 : 0;  // 0: D < near, 1: the rest, 2: all in one
+    if constexpr (!BWD && SEED != kSeedHeap) {
+        if (stage == 2 && walks) {
+            choose_walks();
+            update_H();
+        }
     }
-    for (int q0 = q_first;; q0 += kCols) {
+    float4 nxt[kUnroll];
+    auto first_columns = [&] {
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) {
+            const int q = u * 32 + lane;
+            nxt[u] = q < n4 ? __ldg(row + q) : make_float4(INFINITY, INFINITY, INFINITY, INFINITY);
+        }
+    };
+    first_columns();
+    // kSeedHeap: a pass for the seed columns first
+    for (int q0 = SEED == kSeedHeap ? -kCols : 0;; q0 += kCols) {
         const bool last = q0 >= b.ldc;  // no columns left: empty the queues
         const bool drainall = last || q0 < 0;
         unsigned m16 = 0u;  // bit 4u + e: this lane's column q0 + 128 u + 4 lane + e has D < H
         if (SEED != kSeedHeap || q0 >= 0) {
             // the sign of D - H, first column lowest
-            const float2 nH = make_float2(-H, -H);
+            auto below = [&](float limit) {
+                const float2 nl = make_float2(-limit, -limit);
+                unsigned m = 0u;
 #pragma unroll
-            for (int u = kUnroll - 1; u >= 0; --u) {
-                const float2 hi = add2(make_float2(nxt[u].z, nxt[u].w), nH), lo = add2(make_float2(nxt[u].x, nxt[u].y), nH);
-                m16 = sign_in(sign_in(sign_in(sign_in(m16, hi.y), hi.x), lo.y), lo.x);
-            }
+                for (int u = kUnroll - 1; u >= 0; --u) {
+                    const float2 hi = add2(make_float2(nxt[u].z, nxt[u].w), nl), lo = add2(make_float2(nxt[u].x, nxt[u].y), nl);
+                    m = sign_in(sign_in(sign_in(sign_in(m, hi.y), hi.x), lo.y), lo.x);
+                }
+                return m;
+            };
+            m16 = below(!BWD && stage == 0 ? fminf(H, near) : H);
+            if (!BWD && stage == 1) m16 &= ~below(near);
 #pragma unroll
             for (int u = 0; u < kUnroll; ++u) {
                 const int q = (q0 >> 2) + (kUnroll + u) * 32 + lane;
@@ -388,11 +450,11 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
                     if (q0 + 128 * u + 4 * lane >= b.ldc) m16 &= ~(15u << (4 * u));
             }
             if constexpr (SEED == kSeedHeap) {
-                while (nseed > 0) {
-                    const int i = aux[32 * (kSeedsPerLane - nseed) + lane] - q0;
+                while (nseed < kSeedsPerLane) {
+                    const int i = aux[32 * nseed + lane] - q0;
                     if (i >= kCols) break;
                     m16 &= ~(1u << (4 * (i >> 7) + (i & 3)));
-                    --nseed;
+                    ++nseed;
                 }
             }
         }
@@ -461,35 +523,41 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
                         for (int i = 0; i < kBatch; ++i)
                             if ((pm >> i) & 1u) buf[32 * nb++] = pack_key<BWD>(d[i], col[i]);
                     }
-                    if (__any_sync(kFull, nb > kBuf - kBatch) || (q0 < 0 && qn == 0)) {
-                        const int most = __reduce_max_sync(kFull, nb);
-                        for (int j = 0; j < most; ++j) {
-                            const unsigned long long key = j < nb ? buf[32 * j] : ~0ull;
-                            if (key < heap[0]) sift_down(heap, K, key);
-                        }
-                        nb = 0;
-                        if (lim > -INFINITY) lim = key_dist<BWD>(heap[0]);
-                        update_H();
-                    }
+                    if (__any_sync(kFull, nb > kBuf - kBatch)) flush();
                 }
                 if (!(BWD && SEED == kSeedNone) || an < (last ? 1 : 32)) break;
             }
         }
-        if constexpr (!BWD && SEED == kSeedHeap) {
-            if (q0 < 0 && walks) {
+        if (SEED == kSeedHeap && q0 < 0) {  // the seeds are in
+            flush();
+            if (!BWD) {
+                stage = H > near ? 0 : 2;
+                if (stage == 2 && walks) {
+                    choose_walks();
+                    update_H();
+                }
+            }
+        }
+        if (last) {
+            if (BWD || stage != 0) break;
+            flush();
+            if (walks) {
                 choose_walks();
                 update_H();
             }
+            if (!(H > near)) break;
+            stage = 1;
+            nseed = noseed;
+            q0 = -kCols;
+            first_columns();
         }
-        if (last) break;
     }
 
     // Epilogue: each lane's list in ascending order, padding as (FLT_MAX, 0),
     // the k-th distance for the next backward step, the optional neighbour
     // dump, labels summed in rank order.
     if (!live || ((wide >> lane) & 1u)) return;
-    for (int j = 0; j < nb; ++j)
-        if (buf[32 * j] < heap[0]) sift_down(heap, K, buf[32 * j]);
+    for (int j = 0; j < nb; ++j) enter(buf[32 * j]);
     for (int n = K - 1; n > 0; --n) {
         const unsigned long long end = heap[n * 32];
         heap[n * 32] = heap[0];

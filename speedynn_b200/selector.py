@@ -153,8 +153,8 @@ class Selector:
         check(_lib.lib().snn_set_option(self._h, _lib.SNN_OPT_SORTED_START, int(bool(enable))))
 
     def set_seed_step(self, step):
-        """First forward step whose starting bounds come from seed columns (default 2 for holdout
-        problems with k <= 64, else 1; a large value turns seeded steps off).  Results do not depend on it."""
+        """First forward step whose starting bounds come from seed columns (default: the first
+        that does not run from sorted columns; a large value turns seeded steps off).  Results do not depend on it."""
         check(_lib.lib().snn_set_option(self._h, _lib.SNN_OPT_SEED_STEP, int(step)))
 
     def set_counters(self, enable):
