@@ -154,7 +154,7 @@ cudaError_t launch_walk(const Bufs &b, cudaStream_t s);
 
 // Commit the winner into D (snn_commit.cu); forward commits given seed
 // buffers also keep kSeeds near columns per row for the next step's bounds.
-constexpr int kSeedsPerLane = 8;        // seed columns each lane of the commit keeps
+constexpr int kSeedsPerLane = 8;        // seed columns each lane of the commit keeps: the nearest of each eighth of its columns
 constexpr int kSeeds = 32 * kSeedsPerLane;  // seed columns per row
 cudaError_t launch_commit(const Bufs &b, int backward, int *seeds, float *seed_d, cudaStream_t s);
 

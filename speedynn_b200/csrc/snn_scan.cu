@@ -72,7 +72,7 @@ constexpr float kCap = 0x1.fffffcp+127f;  // largest distance that can enter a l
 // start of a walk, a column of it, a column of another pass over the row (a walk's column: 1.6 instructions, but its gather of D fetches
 // 64 bytes from memory, worth more; fwd-64k 120 ms a selection at 4, 118 at 9).
 constexpr float kQueueCost = 14.0f, kWalkStart = 3000.0f, kWalkCost = 8.0f, kPassCost = 0.2f;
-constexpr int kNear = 1024;  // columns of a row taken first (a power of two times kSeeds)
+static_assert(kSeedsPerLane == 8, "the commit and the scan keep eight seeds per lane");
 static_assert(kQueue >= kSeeds && kQueue >= 128 + 16 + 32, "room for a pass's columns");
 
 // Order-preserving signed key of a float (no NaN), and back.
@@ -168,18 +168,21 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
     const float4 *row = reinterpret_cast<const float4 *>(Dr);
     const int n4 = b.ldc >> 2;
 
-    // near: about the kNear-th smallest committed distance of the row, from the
-    // lanes' 4th and 8th nearest seeds (about the 128th and 256th of the row),
-    // continued as the power law that runs through their means.
+    // near: about the 1,024th smallest committed distance of the row.  A lane's
+    // eight seeds are the minima of eight 256ths of the row, so the middle of them
+    // is about the row's 172nd smallest distance and the largest about the 680th,
+    // by the minimum of m independent values; the power law through the lanes'
+    // means goes on to near (858 to 1,134 columns below it on average in the
+    // steps of the fwd-64k and fwd-200k data).
     float near = INFINITY;
-    auto set_near = [&](float d4, float d8) {
+    auto set_near = [&](float d4, float d5, float d8) {
+        float mid = 0.5f * (d4 + d5);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
-            d4 += __shfl_xor_sync(kFull, d4, o);
+            mid += __shfl_xor_sync(kFull, mid, o);
             d8 += __shfl_xor_sync(kFull, d8, o);
         }
-        float v = d8 * 0.03125f;
-        for (int m = kSeeds; m < kNear; m *= 2) v *= d8 / d4;
+        const float v = d8 * 0.03125f * powf(d8 / mid, 0.298f);  // ln(1024 / 680) / ln(680 / 172)
         if (v < FLT_MAX) near = v;  // otherwise (a lane without eight seeds, ties at 0): one stage for all columns
     };
 
@@ -233,7 +236,7 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
             }
         }
         if (act) lim = fminf(L[SEED - 1], kCap);
-        set_near(__ldg(seed_d + 3 * 32), __ldg(seed_d + 7 * 32));
+        set_near(__ldg(seed_d + 3 * 32), __ldg(seed_d + 4 * 32), __ldg(seed_d + 7 * 32));
     }
 
     // The list starts as K sentinels at the (inclusive) bound, ordered after every
@@ -260,39 +263,45 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
         int si[kSeedsPerLane];
         if (!own) {
             const float *seed_d = b.seed_d + (size_t)r * kSeeds + lane;
-            if (!BWD) set_near(__ldg(seed_d + 3 * 32), __ldg(seed_d + 7 * 32));
+            if (!BWD) set_near(__ldg(seed_d + 3 * 32), __ldg(seed_d + 4 * 32), __ldg(seed_d + 7 * 32));
 #pragma unroll
             for (int j = 0; j < kSeedsPerLane; ++j) si[j] = __ldg(b.seeds + (size_t)r * kSeeds + j * 32 + lane);
         } else {
-            // nobody kept them: the lane's kSeedsPerLane nearest, from a pass of its own
+            // nobody kept them: the same minima from a pass of its own (snn_commit.cu)
             float sv[kSeedsPerLane];
 #pragma unroll
             for (int j = 0; j < kSeedsPerLane; ++j) {
                 sv[j] = INFINITY;
                 si[j] = -1;
             }
-#pragma unroll 1
-            for (int q = lane; q < n4; q += 32) {
-                float4 d = __ldg(row + q);
-#pragma unroll 1
-                for (int e = 0; e < 4; ++e) {
-                    const float v = d.x;
-                    d = make_float4(d.y, d.z, d.w, 0.0f);
-                    if (v < sv[kSeedsPerLane - 1]) {
+            const int part = ((n4 / 2 + 127) / 128) * 128;
 #pragma unroll
-                        for (int j = kSeedsPerLane - 1; j > 0; --j) {
-                            const bool here = v < sv[j], before = v < sv[j - 1];
-                            si[j] = before ? si[j - 1] : here ? 4 * q + e : si[j];
-                            sv[j] = before ? sv[j - 1] : here ? v : sv[j];
-                        }
-                        if (v < sv[0]) {
-                            sv[0] = v;
-                            si[0] = 4 * q + e;
-                        }
+            for (int h = 0; h < 2; ++h) {
+#pragma unroll 4
+                for (int q = h * part + lane; q < (h ? n4 : min(part, n4)); q += 32) {
+                    const float4 d = __ldg(row + q);
+                    const float v[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const bool less = v[e] < sv[4 * h + e];
+                        sv[4 * h + e] = less ? v[e] : sv[4 * h + e];
+                        si[4 * h + e] = less ? 4 * q + e : si[4 * h + e];
                     }
                 }
             }
-            if (!BWD) set_near(sv[3], sv[7]);
+#pragma unroll
+            for (int i = 1; i < kSeedsPerLane; ++i)
+#pragma unroll
+                for (int j = i; j > 0; --j) {
+                    const bool swap = sv[j] < sv[j - 1];
+                    const float lv = swap ? sv[j] : sv[j - 1], hv = swap ? sv[j - 1] : sv[j];
+                    const int li = swap ? si[j] : si[j - 1], hi = swap ? si[j - 1] : si[j];
+                    sv[j - 1] = lv;
+                    sv[j] = hv;
+                    si[j - 1] = li;
+                    si[j] = hi;
+                }
+            if (!BWD) set_near(sv[3], sv[4], sv[7]);
         }
 #pragma unroll
         for (int j = 0; j < kSeedsPerLane; ++j) {  // nearest first

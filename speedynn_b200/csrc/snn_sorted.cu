@@ -84,7 +84,10 @@ __device__ __forceinline__ void insert_idx(int *ix, int n, int v)
     ix[j] = v;
 }
 
-template <int KL>
+// Entries go straight into the label sum in rank order (sequential FP32, as the
+// scoring kernels); only a tie group is held to be put into index order.  (With
+// the whole list in local memory k = 50 took 1.6 ms for 24,989 x 100 problems,
+// now 1.3, and the driver resized the context's local memory for it.)
 __global__ void __launch_bounds__(256) k_first_step(Bufs b, const float *sv, const int *si, int n_cand)
 {
     if (b.st->done) return;
@@ -98,9 +101,21 @@ __global__ void __launch_bounds__(256) k_first_step(Bufs b, const float *sv, con
     const int *bi = si + (size_t)c * b.ldc;
     const float a = b.XV[(size_t)c * b.ldr + r];
 
-    float ld[KL];
-    int li[KL];
+    const size_t o = ((size_t)slot * b.n_rows + r) * K;
+    float acc = 0.0f;
     int cnt = 0;
+    auto take = [&](float d, int i) {  // the next entry of the list
+        if (b.nn_idx) {
+            b.nn_idx[o + cnt] = i;
+            b.nn_dist[o + cnt] = d;
+        }
+        acc = __fadd_rn(acc, __ldg(b.yc + i));
+        ++cnt;
+        for (int m = 0; m < b.nk; ++m) {
+            const int k = __ldg(b.kvals + m);
+            if (k == cnt) b.pred[((size_t)slot * b.nk + m) * b.n_rows + r] = __fdiv_rn(acc, (float)k);
+        }
+    };
     if (isfinite(a)) {
         int lo = 0, hi = n;  // first position with value >= a
         while (lo < hi) {
@@ -115,8 +130,22 @@ __global__ void __launch_bounds__(256) k_first_step(Bufs b, const float *sv, con
         while (cnt < K) {
             const float dm = fminf(dl, dr);
             if (!(dm < FLT_MAX)) break;
-            int g = 0;
+            const bool from_left = dl == dm;
+            const int first = from_left ? bi[L] : bi[R];
+            if (from_left) {
+                --L;
+                dl = L >= 0 ? dist1(a, bv[L]) : INFINITY;
+            } else {
+                ++R;
+                dr = R < n ? dist1(a, bv[R]) : INFINITY;
+            }
+            if (dl != dm && dr != dm) {  // the usual case: nothing at the same distance
+                take(dm, first);
+                continue;
+            }
+            int g = 1;
             bool over = false;
+            tie[0] = first;
             while (L >= 0 && dl == dm) {  // the group's run on the left
                 if (g < kTieCap) insert_idx(tie, g, bi[L]);
                 else over = true;
@@ -135,33 +164,10 @@ __global__ void __launch_bounds__(256) k_first_step(Bufs b, const float *sv, con
                 atomicExch(&b.st->full_scan, 1);
                 return;
             }
-            for (int j = 0; j < g && cnt < K; ++j) {
-                ld[cnt] = dm;
-                li[cnt] = tie[j];
-                ++cnt;
-            }
+            for (int j = 0; j < g && cnt < K; ++j) take(dm, tie[j]);
         }
     }
-    for (int j = cnt; j < K; ++j) {
-        ld[j] = FLT_MAX;
-        li[j] = 0;
-    }
-    if (b.nn_idx) {
-        const size_t o = ((size_t)slot * b.n_rows + r) * K;
-        for (int j = 0; j < K; ++j) {
-            b.nn_idx[o + j] = li[j];
-            b.nn_dist[o + j] = ld[j];
-        }
-    }
-    // labels summed in rank order (sequential FP32), as the scoring kernels
-    float acc = 0.0f;
-    for (int j = 0; j < K; ++j) {
-        acc = __fadd_rn(acc, __ldg(b.yc + li[j]));
-        for (int m = 0; m < b.nk; ++m) {
-            const int k = __ldg(b.kvals + m);
-            if (k == j + 1) b.pred[((size_t)slot * b.nk + m) * b.n_rows + r] = __fdiv_rn(acc, (float)k);
-        }
-    }
+    while (cnt < K) take(FLT_MAX, 0);  // padding
 }
 
 // k_second_step: the second forward step of a holdout problem.  With one
@@ -656,9 +662,7 @@ cudaError_t launch_walk(const Bufs &b, cudaStream_t s)
 cudaError_t launch_first_step(const Bufs &b, const float *sv, const int *si, int n_cand, cudaStream_t s)
 {
     const dim3 grid((b.n_rows + 255) / 256, n_cand);
-    if (b.kmax <= 16) k_first_step<16><<<grid, 256, 0, s>>>(b, sv, si, n_cand);
-    else if (b.kmax <= 64) k_first_step<64><<<grid, 256, 0, s>>>(b, sv, si, n_cand);
-    else k_first_step<kScoreMaxK><<<grid, 256, 0, s>>>(b, sv, si, n_cand);
+    k_first_step<<<grid, 256, 0, s>>>(b, sv, si, n_cand);
     return cudaGetLastError();
 }
 
