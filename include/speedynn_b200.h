@@ -316,7 +316,8 @@ SNN_API int snn_batch_destroy(snn_batch *b);
  * greedy step from caller-owned DEVICE buffers and writes every candidate's
  * RMSE for every k: errors[c * num_k_vals + m] (FP32, the reference's value)
  * and errors64 (same residuals summed in FP64).  It never allocates: its
- * scratch (kNN predictions, step state, copies of cands and k_vals) is a
+ * scratch (kNN predictions, step state, copies of cands and k_vals, and a
+ * forward step's packed candidates where they fit) is a
  * fixed 16 MB static device array, so n_cand * num_k_vals * n_rows must not
  * exceed 4,194,304 (else SNN_ERR_ARG), num_k_vals <= 256, n_cand <= 1024.
  *

@@ -106,6 +106,7 @@ struct snn_handle {
     float *xg = nullptr;          // pruned scan: packed candidates [ceil(p / 32)][ldc][32]
     float2 *ext = nullptr;        // backward: [ceil(p / 32)][ldc] column extremes
     float4 *fstat = nullptr;      // backward: per-feature mean and range
+    int bwd_dense = 0;            // backward: 1 the dense scorer is faster on the loaded data, -1 not known (probe each step)
     int *walk = nullptr, *n_walk = nullptr;  // forward holdout: problems left to k_walk, and how many
     bool sorted_start = true;     // SNN_OPT_SORTED_START
     bool seeds_ok = false;        // seeds hold the current D's seed columns
@@ -337,7 +338,7 @@ constexpr int kScanAllCols = 4096;
 int scan_seeding(const snn_handle *h, int t, bool seeded)
 {
     if (h->kernel != 0 || h->count_filter || h->inject_stall >= 0) return -1;
-    if (h->desc.backward) return h->prev_ok ? snn::kNoSeeds : snn::kOwnSeeds;
+    if (h->desc.backward) return h->bwd_dense == 1 ? -1 : h->prev_ok ? snn::kNoSeeds : snn::kOwnSeeds;
     if (seeded) return snn::kGivenSeeds;
     return t == 0 && h->n_cols <= kScanAllCols ? snn::kOwnSeeds : -1;
 }
@@ -378,10 +379,22 @@ int issue_step(snn_handle *h, int t)
         h->n_launch += dense_seeded ? 2 : 1;
     }
     if (scan) {
-        SNN_CUDA(snn::launch_scan(b, n_cand, backward, seeding, h->max_smem, h->stream));
+        // Forward, distances over one to three two-valued features leave most columns
+        // open (30,000 x 15,000 x 40 such features, second step: 23.7 ms, dense 8.3);
+        // the probe and the launch that returns at once take 0.1 ms of a fwd-64k step.
+        const bool gated = (backward ? h->bwd_dense < 0 : t <= 3) && snn::scan_worth_probing(b, n_cand);
+        if (gated) SNN_CUDA(snn::launch_scan_probe(b, n_cand, backward, seeding, h->max_smem, h->stream));
+        SNN_CUDA(snn::launch_scan(b, n_cand, backward, seeding, gated, h->max_smem, h->stream));
         if (snn::scan_leaves_walks(b, n_cand, backward)) {
             SNN_CUDA(snn::launch_walk(b, h->stream));
             h->n_launch += 1;
+        }
+        if (gated) {  // usually returns at once
+            Bufs d = b;
+            d.only_if_full = 1;
+            d.use_prev = seeding == snn::kNoSeeds ? 1 : 0;
+            SNN_CUDA(snn::launch_score_tma(d, n_cand, backward, h->stream));  // k <= 64 (scan_worth_probing)
+            h->n_launch += 1 + snn::score_tma_launches(h->kmax, n_cand, backward);
         }
         prev = backward;
     } else if (use_tma(h)) {
@@ -694,6 +707,25 @@ static int load_impl(snn_handle *h, const float *X_train, const float *y_train, 
     h->loaded = true;
     reset_timing(h);
     if (int rc = issue_reset(h)) return rc;
+    // Backward, whether pruning pays depends on the data (on features of very
+    // different reach it does not: 30,000 x 15,000 x 40 log-normal columns 131 ms a
+    // run pruned, 55 dense; normal ones 41 against 44): a probe of the full
+    // distances decides for the runs on this data, before the wait at the end of
+    // the load.  A batch does not wait here; its steps probe by themselves.
+    h->bwd_dense = 0;
+    if (h->desc.backward && h->kernel == 0 && snn::scan_worth_probing(h->bufs(), h->p)) {
+        h->bwd_dense = -1;
+        if (wait) {
+            const Bufs b = h->bufs();
+            State s;
+            SNN_CUDA(snn::launch_pack_groups(b, h->p, 1, h->stream));
+            SNN_CUDA(snn::launch_scan_probe(b, h->p, 1, snn::kOwnSeeds, h->max_smem, h->stream));
+            if (int rc = read_state(h, &s)) return rc;
+            h->bwd_dense = s.full_scan;
+            if (s.full_scan || s.flat)  // the step starts with a clear state
+                SNN_CUDA(snn::launch_reset_state(b, 1, h->total_steps, h->stream));
+        }
+    }
     // A batch issues the selection on the same stream right away (its inputs
     // stay valid until the batch run returns); a single load waits, so the
     // caller may reuse pinned source buffers at once.

@@ -41,7 +41,8 @@ struct State {
     int n_cand;       // candidates of the next step
     int best_k_last;  // best k of the last winner
     int num_final;    // features in the model after the last step
-    int full_scan;    // 1: the sorted first step left problems to the full scan (snn_sorted.cu)
+    int full_scan;    // 1: the sorted first steps or the pruned scan leave the step to the dense scorer
+    int flat;         // the pruned scan's probe in this step: warps << 20, their estimated cost
 };
 
 // Everything a kernel needs, passed by value.
@@ -110,7 +111,7 @@ struct Bufs {
     int *n_walk;
     const float *sval;
     const int *sidx;
-    int only_if_full;  // scoring kernels return at once unless st->full_scan is set (sorted first step)
+    int only_if_full;  // scoring kernels return at once unless st->full_scan is set
 };
 
 constexpr int kPadCols = 64;     // row stride multiple of the feature-major arrays / D
@@ -147,9 +148,14 @@ enum { kNoSeeds = 0, kGivenSeeds = 1, kOwnSeeds = 2 };
 inline int scan_groups(int n_cand) { return (n_cand + 31) / 32; }  // groups of at most 32 candidates
 inline int scan_group_size(int n_cand) { return (n_cand + scan_groups(n_cand) - 1) / scan_groups(n_cand); }  // of a full group
 cudaError_t launch_pack_groups(const Bufs &b, int n_cand, int backward, cudaStream_t s);
-// May leave problems in b.walk for launch_walk (scan_leaves_walks).
-cudaError_t launch_scan(const Bufs &b, int n_cand, int backward, int seeding, int max_smem, cudaStream_t s);
+// May leave problems in b.walk for launch_walk (scan_leaves_walks).  gated: does
+// nothing if State::full_scan is set (the dense scorer follows with only_if_full).
+cudaError_t launch_scan(const Bufs &b, int n_cand, int backward, int seeding, bool gated, int max_smem, cudaStream_t s);
 bool scan_leaves_walks(const Bufs &b, int n_cand, int backward);
+// Estimates from a few rows what the scan would cost and sets State::full_scan
+// if the dense scorer is faster; for problems where it may be (scan_worth_probing).
+cudaError_t launch_scan_probe(const Bufs &b, int n_cand, int backward, int seeding, int max_smem, cudaStream_t s);
+bool scan_worth_probing(const Bufs &b, int n_cand);
 cudaError_t launch_walk(const Bufs &b, cudaStream_t s);
 
 // Commit the winner into D (snn_commit.cu); forward commits given seed

@@ -287,6 +287,8 @@ __global__ void __launch_bounds__(32) k_select(Bufs b, int n_cand, int it, int t
         b.err_all[l * b.p + it] = b.lossval[((size_t)l * n_cand + wi) * b.nk + wm];
     next_candidates(b, wdim, backward);
     if (lane != 0) return;
+    st->full_scan = 0;
+    st->flat = 0;
     const int wk = b.kvals[wm];
     st->winner = wdim;
     b.order[it] = wdim;
@@ -347,6 +349,7 @@ __global__ void k_reset_state(Bufs b, int backward, int total_steps)
         s.best_k_last = 0;
         s.num_final = backward ? b.p : 0;
         s.full_scan = 0;
+        s.flat = 0;
         *b.st = s;
     }
 }

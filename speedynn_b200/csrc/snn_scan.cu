@@ -72,6 +72,10 @@ constexpr float kCap = 0x1.fffffcp+127f;  // largest distance that can enter a l
 // start of a walk, a column of it, a column of another pass over the row (a walk's column: 1.6 instructions, but its gather of D fetches
 // 64 bytes from memory, worth more; fwd-64k 120 ms a selection at 4, 118 at 9).
 constexpr float kQueueCost = 14.0f, kWalkStart = 3000.0f, kWalkCost = 8.0f, kPassCost = 0.2f;
+// Per column of a group: reading it, the second test, and the dense scorers' work
+// per candidate (measured: 30,000 x 15,000 x 38 8 ms, the scan 14 with 68 % open).
+constexpr float kReadCost = 0.25f, kTestCost = 4.0f, kDenseCost = 0.28f;
+constexpr int kProbeRows = 64;
 static_assert(kSeedsPerLane == 8, "the commit and the scan keep eight seeds per lane");
 static_assert(kQueue >= kSeeds && kQueue >= 128 + 16 + 32, "room for a pass's columns");
 
@@ -119,10 +123,10 @@ __device__ __forceinline__ void sift_down(unsigned long long *h, int n, unsigned
     h[i * 32] = key;
 }
 
-// Shared memory of a warp: heaps and buffers (two batches) of 32 lanes, one or two lists of columns.
-size_t warp_smem(int K, int batch, bool aux)
+// Shared memory of a warp: heaps and buffers (two batches) of 32 lanes, and lists of columns.
+size_t warp_smem(int K, int batch, int lists)
 {
-    return sizeof(unsigned long long) * 32 * (size_t)(K + 2 * batch) + sizeof(int) * (size_t)kQueue * (aux ? 2 : 1);
+    return sizeof(unsigned long long) * 32 * (size_t)(K + 2 * batch) + sizeof(int) * (size_t)kQueue * lists;
 }
 
 __device__ __forceinline__ unsigned sign_in(unsigned m, float v) { return __funnelshift_l(__float_as_uint(v), m, 1); }
@@ -143,18 +147,21 @@ constexpr int kSeedNone = 0, kSeedHeap = -1;
 constexpr int kBatchMany = 4, kBatchFew = 16, kWarpsMany = 28;
 
 template <bool BWD, int SEED, int kBatch>
-__global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_scan(Bufs b, int n_cand, int G, int gs, int walks, int own)
+__global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_scan(Bufs b, int n_cand, int G, int gs, int walks, int own, int gated, int probe)
 {
     constexpr int kBuf = 2 * kBatch;
     extern __shared__ __align__(16) unsigned char smraw[];
     if (b.st->done) return;
+    if (gated && b.st->full_scan) return;  // the dense scorer takes the step
     const int lane = threadIdx.x;  // blocks of one warp: warps finish at different times
-    const int r = blockIdx.x / G, g = blockIdx.x % G;
+    // probe: only estimate, for rows that far apart, what the scan would cost
+    const int r = blockIdx.x / G * (probe ? probe : 1), g = blockIdx.x % G;
     const int K = b.kmax;
     unsigned long long *heap = reinterpret_cast<unsigned long long *>(smraw) + lane;
     unsigned long long *buf = heap + (size_t)K * 32;
     int *queue = reinterpret_cast<int *>(smraw + sizeof(unsigned long long) * 32 * (size_t)(K + kBuf));
-    int *aux = queue + kQueue;  // backward: columns before the second test; kSeedHeap: the lanes' seed columns
+    int *wait = queue + kQueue;                  // backward: columns before the second test
+    int *own_seed = queue + (BWD ? 2 : 1) * kQueue;  // kSeedHeap: the lanes' seed columns
 
     const int slot = g * gs + lane;
     const bool live = lane < gs && slot < n_cand;
@@ -257,8 +264,8 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
     // kSeedHeap: the seed columns go through the queue before the row's others; the
     // lane keeps its own (the commit and this kernel give each lane the same
     // columns), ascending, to leave them out afterwards.
-    int nseed = 0;  // the lane's seed columns already passed, the next at aux[32 * nseed + lane]
-    int noseed = 0;  // entries of aux without a column
+    int nseed = 0;  // the lane's seed columns already passed, the next at own_seed[32 * nseed + lane]
+    int noseed = 0;  // entries of own_seed without a column
     if constexpr (SEED == kSeedHeap) {
         int si[kSeedsPerLane];
         if (!own) {
@@ -320,7 +327,7 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
                 si[j] = hi;
             }
 #pragma unroll
-        for (int j = 0; j < kSeedsPerLane; ++j) aux[32 * j + lane] = si[j];
+        for (int j = 0; j < kSeedsPerLane; ++j) own_seed[32 * j + lane] = si[j];
     }
 
     // Backward: each candidate's largest possible square on this row and the
@@ -355,6 +362,18 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
         }
     };
     unsigned wide = 0u;  // forward: candidates left to k_walk, their lim -inf here
+    // probe: the group's estimated instructions against the dense scorer's.  Where
+    // most columns stay open (distances that hardly differ, as with two-valued
+    // features committed; backward, features whose squares reach far) that one is
+    // faster; the last of the probing warps decides, at ten sixteenths since ties make
+    // a queued column dearer than estimated.
+    auto vote = [&](float cost) {
+        if (lane != 0) return;
+        const float dense = kDenseCost * (float)gs * (K <= 16 ? 1.0f : K <= 32 ? 1.5f : 2.0f) * (float)b.n_cols;
+        const int units = (int)fminf(16.0f * cost / dense, 64.0f);
+        const int old = atomicAdd(&b.st->flat, (1 << 20) + units);
+        if ((old >> 20) + 1 == (int)gridDim.x && (old & 0xfffff) + units > 10 * (int)gridDim.x) b.st->full_scan = 1;
+    };
     auto choose_walks = [&] {
         // The split with the least estimated cost, from 128 sampled columns (64 for
         // the candidates' own squares): a queued column costs the group kQueueCost
@@ -367,24 +386,33 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
             const float smp = __ldg(Dr + j0 + lane);
 #pragma unroll 8
             for (int l = 0; l < 32; ++l) cd += __shfl_sync(kFull, smp, l) <= lim ? 1 : 0;
+            if (walks) {
 #pragma unroll 8
-            for (int l = 0; l < 16; ++l) {
-                const float t = xv - __ldg(xg + (size_t)(j0 + l) * 32);
-                cs += t * t <= lim ? 1 : 0;
+                for (int l = 0; l < 16; ++l) {
+                    const float t = xv - __ldg(xg + (size_t)(j0 + l) * 32);
+                    cs += t * t <= lim ? 1 : 0;
+                }
             }
         }
         const float n = (float)b.n_cols;
-        const int walk = (int)(kWalkStart + kWalkCost / 64.0f * n * (float)cs);
         // if the candidates with more columns walk; beyond near the row is read once more
-        int cost = (int)(kQueueCost / 128.0f * n * (float)cd + (lim >= near ? kPassCost * n : 0.0f));
+        float cost = kQueueCost / 128.0f * n * (float)cd + (lim >= near ? kPassCost * n : 0.0f);
+        if (walks) {
+            const float walk = kWalkStart + kWalkCost / 64.0f * n * (float)cs;
 #pragma unroll 4
-        for (int l = 0; l < 32; ++l) {
-            const int wl = __shfl_sync(kFull, walk, l), cl = __shfl_sync(kFull, cd, l);
-            cost += cl > cd ? wl : 0;
+            for (int l = 0; l < 32; ++l) {
+                const float wl = __shfl_sync(kFull, walk, l);
+                cost += __shfl_sync(kFull, cd, l) > cd ? wl : 0.0f;
+            }
         }
-        const int best = __reduce_min_sync(kFull, cost);
-        const int cut = __reduce_min_sync(kFull, cost == best ? cd : 999);
-        wide = __ballot_sync(kFull, cd > cut);
+        // positive: the bits order like the values
+        const int best = walks ? __reduce_min_sync(kFull, __float_as_int(cost)) : __reduce_max_sync(kFull, __float_as_int(cost));
+        if (probe) {  // the near columns, taken first, at least halve what stays open (mixture-50k: a quarter)
+            vote(__int_as_float(best) * (H > near ? 0.5f : 1.0f));
+            return;
+        }
+        const int cut = __reduce_min_sync(kFull, __float_as_int(cost) == best ? cd : 999);
+        wide = walks ? __ballot_sync(kFull, cd > cut) : 0u;
         if (wide) {
             int at = 0;
             if (lane == 0) at = atomicAdd(b.n_walk, __popc(wide));
@@ -396,9 +424,23 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
             }
         }
     };
+    // Backward's probe, lane = column: sampled columns queued, and kept by the second test.
+    auto probe_backward = [&] {
+        int c1 = 0, c2 = 0;
+        for (int i = 0; i < 4; ++i) {
+            const int j = i * (b.n_cols / 4) + lane;
+            const float D = __ldg(Dr + j);
+            const float2 x = __ldg(b.ext + (size_t)g * b.ldc + j);
+            const float U = fmaxf(__fsub_ru(amax, x.x), __fsub_ru(x.y, amin));
+            const bool q = D < H;
+            c1 += __popc(__ballot_sync(kFull, q));
+            c2 += __popc(__ballot_sync(kFull, q && __fsub_rn(D, __fmul_rn(U, U)) <= kmx));
+        }
+        vote((float)b.n_cols * (kReadCost + kTestCost / 128.0f * (float)c1 + kQueueCost / 128.0f * (float)c2));
+    };
 
     int nb = 0;  // the lane's buffered keys
-    int ah = 0, an = 0;  // backward: columns that wait for the second test (aux)
+    int ah = 0, an = 0;  // backward: columns that wait for the second test
     auto flush = [&] {
         const int most = __reduce_max_sync(kFull, nb);
         for (int j = 0; j < most; ++j) {
@@ -414,11 +456,14 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
     // first, which leaves nearly exact bounds for the split and for the others
     // (or none of them open).
     int stage = BWD || !(H > near) ? 2 : 0;  // 0: D < near, 1: the rest, 2: all in one
-    if constexpr (!BWD && SEED != kSeedHeap) {
-        if (stage == 2 && walks) {
+    if constexpr (SEED != kSeedHeap) {
+        if constexpr (BWD) {
+            if (probe) probe_backward();
+        } else if (probe || (stage == 2 && walks)) {
             choose_walks();
             update_H();
         }
+        if (probe) return;
     }
     float4 nxt[kUnroll];
     auto first_columns = [&] {
@@ -460,7 +505,7 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
             }
             if constexpr (SEED == kSeedHeap) {
                 while (nseed < kSeedsPerLane) {
-                    const int i = aux[32 * nseed + lane] - q0;
+                    const int i = own_seed[32 * nseed + lane] - q0;
                     if (i >= kCols) break;
                     m16 &= ~(1u << (4 * (i >> 7) + (i & 3)));
                     ++nseed;
@@ -478,22 +523,22 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
                     mp &= mp - 1;
                     const int at = __popc(any & ((1u << lane) - 1u));
                     const int col = q0 + 128 * (i >> 2) + 4 * lane + (i & 3);
-                    if constexpr (BWD && SEED == kSeedNone) aux[(ah + an + at) & (kQueue - 1)] = col;
+                    if constexpr (BWD) wait[(ah + an + at) & (kQueue - 1)] = col;
                     else queue[(qh + qn + at) & (kQueue - 1)] = col;
                 }
-                if constexpr (BWD && SEED == kSeedNone) an += __popc(any);
+                if constexpr (BWD) an += __popc(any);
                 else qn += __popc(any);
             }
             __syncwarp();
             for (;;) {
-                if constexpr (BWD && SEED == kSeedNone) {
+                if constexpr (BWD) {
                     if (an >= (last ? 1 : 32)) {
                         // Second test, lane = column: an s of this column is at most U^2, U the
                         // larger of the two extreme differences (rounded up), so an entry needs
                         // D - fl(U^2) < nextafter(lim) for some candidate, and its rounding <= kmx.
                         const int n = min(an, 32);
                         const bool in = lane < n;
-                        const int col = in ? aux[(ah + lane) & (kQueue - 1)] : 0;
+                        const int col = in ? wait[(ah + lane) & (kQueue - 1)] : 0;
                         const float D = __ldg(Dr + col);
                         const float2 x = __ldg(b.ext + (size_t)g * b.ldc + col);
                         const float U = fmaxf(__fsub_ru(amax, x.x), __fsub_ru(x.y, amin));
@@ -534,18 +579,21 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
                     }
                     if (__any_sync(kFull, nb > kBuf - kBatch)) flush();
                 }
-                if (!(BWD && SEED == kSeedNone) || an < (last ? 1 : 32)) break;
+                if (!BWD || an < (last ? 1 : 32)) break;
             }
         }
         if (SEED == kSeedHeap && q0 < 0) {  // the seeds are in
             flush();
-            if (!BWD) {
+            if constexpr (BWD) {
+                if (probe) probe_backward();
+            } else {
                 stage = H > near ? 0 : 2;
-                if (stage == 2 && walks) {
+                if (probe || (stage == 2 && walks)) {
                     choose_walks();
                     update_H();
                 }
             }
+            if (probe) return;
         }
         if (last) {
             if (BWD || stage != 0) break;
@@ -645,34 +693,67 @@ int sm_count_scan()
     return n;
 }
 
-template <bool BWD, int SEED, int BATCH>
-cudaError_t launch_batch(const Bufs &b, int n_cand, bool own, int max_smem, cudaStream_t s)
+// At most one wave of warps: a warp's chain of work is the kernel's time.
+bool one_wave(const Bufs &b, int n_cand)
 {
-    const int G = scan_groups(n_cand), gs = scan_group_size(n_cand);
-    const size_t smem = warp_smem(b.kmax, BATCH, BWD || SEED == kSeedHeap);
-    const long long blocks = (long long)b.n_rows * G;
-    if (smem > (size_t)max_smem || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    const int walks = scan_leaves_walks(b, n_cand, BWD);
-    if (walks) {
-        const cudaError_t e = cudaMemsetAsync(b.n_walk, 0, sizeof(int), s);
+    return (long long)b.n_rows * scan_groups(n_cand) <= (long long)sm_count_scan() * kWarpsMany;
+}
+
+struct ScanCall {
+    int n_cand;
+    bool own;       // the kernel finds the seed columns itself
+    bool gated;     // return at once if State::full_scan is set
+    bool probe;     // only the probe's estimate
+    int max_smem;
+    cudaStream_t stream;
+};
+
+template <bool BWD, int SEED, int BATCH>
+cudaError_t launch_batch(const Bufs &b, const ScanCall &c)
+{
+    const int G = scan_groups(c.n_cand), gs = scan_group_size(c.n_cand);
+    const size_t smem = warp_smem(b.kmax, BATCH, 1 + (BWD ? 1 : 0) + (SEED == kSeedHeap ? 1 : 0));
+    const long long blocks = (long long)(c.probe ? kProbeRows : b.n_rows) * G;
+    if (smem > (size_t)c.max_smem || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+    const int walks = scan_leaves_walks(b, c.n_cand, BWD);
+    if (walks && !c.probe) {
+        const cudaError_t e = cudaMemsetAsync(b.n_walk, 0, sizeof(int), c.stream);
         if (e != cudaSuccess) return e;
     }
     auto kern = k_scan<BWD, SEED, BATCH>;
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kern<<<(unsigned)blocks, 32, smem, s>>>(b, n_cand, G, gs, walks, own ? 1 : 0);
+    kern<<<(unsigned)blocks, 32, smem, c.stream>>>(b, c.n_cand, G, gs, walks, c.own ? 1 : 0, c.gated ? 1 : 0,
+                                                   c.probe ? b.n_rows / kProbeRows : 0);
     return cudaGetLastError();
 }
 
 template <bool BWD, int SEED>
-cudaError_t launch_seeded(const Bufs &b, int n_cand, bool own, int max_smem, cudaStream_t s)
+cudaError_t launch_seeded(const Bufs &b, const ScanCall &c)
 {
-    const long long warps = (long long)b.n_rows * scan_groups(n_cand);
-    if (warps <= (long long)sm_count_scan() * kWarpsMany) return launch_batch<BWD, SEED, kBatchFew>(b, n_cand, own, max_smem, s);
-    return launch_batch<BWD, SEED, kBatchMany>(b, n_cand, own, max_smem, s);
+    return one_wave(b, c.n_cand) ? launch_batch<BWD, SEED, kBatchFew>(b, c) : launch_batch<BWD, SEED, kBatchMany>(b, c);
+}
+
+cudaError_t launch_any(const Bufs &b, int backward, int seeding, const ScanCall &c)
+{
+    if (backward) return seeding == kNoSeeds ? launch_seeded<true, kSeedNone>(b, c) : launch_seeded<true, kSeedHeap>(b, c);
+    // lists of up to 16: bounds from group minima; longer ones start from the seeds themselves
+    if (c.own || b.kmax > 16) return launch_seeded<false, kSeedHeap>(b, c);
+    if (b.kmax <= 8) return launch_seeded<false, 8>(b, c);
+    if (b.kmax <= 12) return launch_seeded<false, 12>(b, c);
+    return launch_seeded<false, 16>(b, c);
 }
 
 }  // namespace
+
+// One wave of warps gains from pruning even if every column is open (its time
+// is one warp's chain of work: step 1 of a 3000-row CV problem, everything
+// open, 0.36 against 0.58 ms), and lists above 64 have no dense scorer that
+// comes near.
+bool scan_worth_probing(const Bufs &b, int n_cand)
+{
+    return b.kmax <= 64 && b.n_cols >= 1024 && b.n_rows >= kProbeRows && !one_wave(b, n_cand);
+}
 
 bool scan_leaves_walks(const Bufs &b, int n_cand, int backward)
 {
@@ -685,18 +766,14 @@ cudaError_t launch_pack_groups(const Bufs &b, int n_cand, int backward, cudaStre
     return cudaGetLastError();
 }
 
-cudaError_t launch_scan(const Bufs &b, int n_cand, int backward, int seeding, int max_smem, cudaStream_t s)
+cudaError_t launch_scan(const Bufs &b, int n_cand, int backward, int seeding, bool gated, int max_smem, cudaStream_t s)
 {
-    const bool own = seeding == kOwnSeeds;
-    if (backward) {
-        if (seeding == kNoSeeds) return launch_seeded<true, kSeedNone>(b, n_cand, false, max_smem, s);
-        return launch_seeded<true, kSeedHeap>(b, n_cand, true, max_smem, s);
-    }
-    // lists of up to 16: bounds from group minima; longer ones start from the seeds themselves
-    if (own || b.kmax > 16) return launch_seeded<false, kSeedHeap>(b, n_cand, own, max_smem, s);
-    if (b.kmax <= 8) return launch_seeded<false, 8>(b, n_cand, false, max_smem, s);
-    if (b.kmax <= 12) return launch_seeded<false, 12>(b, n_cand, false, max_smem, s);
-    return launch_seeded<false, 16>(b, n_cand, false, max_smem, s);
+    return launch_any(b, backward, seeding, {n_cand, seeding == kOwnSeeds, gated, false, max_smem, s});
+}
+
+cudaError_t launch_scan_probe(const Bufs &b, int n_cand, int backward, int seeding, int max_smem, cudaStream_t s)
+{
+    return launch_any(b, backward, seeding, {n_cand, seeding == kOwnSeeds, false, true, max_smem, s});
 }
 
 }  // namespace snn

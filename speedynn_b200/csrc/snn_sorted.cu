@@ -595,7 +595,7 @@ __global__ void __launch_bounds__(256, 8) k_second_step_long(Bufs b, const float
 // in flight.
 __global__ void __launch_bounds__(256, 4) k_walk(Bufs b)
 {
-    if (b.st->done) return;
+    if (b.st->done || b.st->full_scan) return;
     const int total = *b.n_walk;
     for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < total; i += gridDim.x * (blockDim.x >> 5)) {
         const int slot = b.walk[i] / b.n_rows, r = b.walk[i] % b.n_rows;
