@@ -145,21 +145,31 @@ constexpr int kSeedNone = 0, kSeedHeap = -1;
 // problems of at most one such wave of warps, whose time is the chain of
 // gathers of one warp, take batches of 16.
 constexpr int kBatchMany = 4, kBatchFew = 16, kWarpsMany = 28;
+// ... and, forward from given bounds, two warps for each (row, group), each with
+// every other pass over the row; the first one merges the lists (steps 3 to 8 of
+// 2,000 x 1,000 x 20: 0.50 -> 0.39 ms; four warps 0.45; backward, where the work
+// before the lists is short, it loses: 1,501 x 14 1.35 -> 1.50 ms a run).
+constexpr int kMaxSplit = 2;
 
 template <bool BWD, int SEED, int kBatch>
-__global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_scan(Bufs b, int n_cand, int G, int gs, int walks, int own, int gated, int probe)
+__global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit, kBatch == kBatchMany ? kWarpsMany : 16 / kMaxSplit)
+    k_scan(Bufs b, int n_cand, int G, int gs, int walks, int own, int gated, int probe)
 {
     constexpr int kBuf = 2 * kBatch;
     extern __shared__ __align__(16) unsigned char smraw[];
     if (b.st->done) return;
     if (gated && b.st->full_scan) return;  // the dense scorer takes the step
-    const int lane = threadIdx.x;  // blocks of one warp: warps finish at different times
+    constexpr bool kSplit = kBatch == kBatchFew && SEED > 0;
+    // blocks of one warp for many: warps finish at different times
+    const int lane = threadIdx.x & 31, w = kSplit ? threadIdx.x >> 5 : 0, warps = kSplit ? blockDim.x >> 5 : 1;
     // probe: only estimate, for rows that far apart, what the scan would cost
     const int r = blockIdx.x / G * (probe ? probe : 1), g = blockIdx.x % G;
     const int K = b.kmax;
-    unsigned long long *heap = reinterpret_cast<unsigned long long *>(smraw) + lane;
+    const size_t lists_at = sizeof(unsigned long long) * 32 * (size_t)(K + kBuf);
+    const size_t wsmem = lists_at + sizeof(int) * kQueue;  // of a warp, where there are several
+    unsigned long long *heap = reinterpret_cast<unsigned long long *>(smraw + w * wsmem) + lane;
     unsigned long long *buf = heap + (size_t)K * 32;
-    int *queue = reinterpret_cast<int *>(smraw + sizeof(unsigned long long) * 32 * (size_t)(K + kBuf));
+    int *queue = reinterpret_cast<int *>(smraw + w * wsmem + lists_at);
     int *wait = queue + kQueue;                  // backward: columns before the second test
     int *own_seed = queue + (BWD ? 2 : 1) * kQueue;  // kSeedHeap: the lanes' seed columns
 
@@ -251,12 +261,13 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
     // They give way from the last entry up, where a key sinks through few levels
     // or none; once all are gone (put is 0), a key replaces the largest entry.
     for (int j = 0; j < K; ++j) heap[j * 32] = pack_key<BWD>(lim, -1);
-    // (Not beside the second test, whose registers are all in use.)
-    int put = BWD && SEED == kSeedNone ? 0 : K - 1;
+    // (Not in the large backward instance, whose registers are all in use.)
+    constexpr bool kPut = !(BWD && SEED == kSeedNone && kBatch == kBatchMany);
+    int put = kPut ? K - 1 : 0;
     auto enter = [&](unsigned long long key) {
         if (key < heap[put * 32]) {
             sift_down(heap, K, key, put);
-            if (!(BWD && SEED == kSeedNone)) put = max(put - 1, 0);
+            if (kPut) put = max(put - 1, 0);
         }
     };
 
@@ -469,13 +480,13 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
     auto first_columns = [&] {
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u) {
-            const int q = u * 32 + lane;
+            const int q = w * (kCols / 4) + u * 32 + lane;
             nxt[u] = q < n4 ? __ldg(row + q) : make_float4(INFINITY, INFINITY, INFINITY, INFINITY);
         }
     };
     first_columns();
     // kSeedHeap: a pass for the seed columns first
-    for (int q0 = SEED == kSeedHeap ? -kCols : 0;; q0 += kCols) {
+    for (int q0 = SEED == kSeedHeap ? -kCols : w * kCols;; q0 += warps * kCols) {
         const bool last = q0 >= b.ldc;  // no columns left: empty the queues
         const bool drainall = last || q0 < 0;
         unsigned m16 = 0u;  // bit 4u + e: this lane's column q0 + 128 u + 4 lane + e has D < H
@@ -495,7 +506,7 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
             if (!BWD && stage == 1) m16 &= ~below(near);
 #pragma unroll
             for (int u = 0; u < kUnroll; ++u) {
-                const int q = (q0 >> 2) + (kUnroll + u) * 32 + lane;
+                const int q = (q0 >> 2) + (kUnroll * warps + u) * 32 + lane;
                 nxt[u] = q < n4 ? __ldg(row + q) : make_float4(INFINITY, INFINITY, INFINITY, INFINITY);
             }
             if (q0 + kCols > b.ldc) {  // past the row
@@ -605,7 +616,7 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
             if (!(H > near)) break;
             stage = 1;
             nseed = noseed;
-            q0 = -kCols;
+            q0 = (w - warps) * kCols;
             first_columns();
         }
     }
@@ -613,8 +624,21 @@ __global__ void __launch_bounds__(32, kBatch == kBatchMany ? kWarpsMany : 16) k_
     // Epilogue: each lane's list in ascending order, padding as (FLT_MAX, 0),
     // the k-th distance for the next backward step, the optional neighbour
     // dump, labels summed in rank order.
-    if (!live || ((wide >> lane) & 1u)) return;
     for (int j = 0; j < nb; ++j) enter(buf[32 * j]);
+    if constexpr (kSplit) {
+        if (warps > 1) {
+            __syncthreads();
+            if (w > 0) return;
+            for (int v = 1; v < warps; ++v) {
+                const unsigned long long *other = reinterpret_cast<const unsigned long long *>(smraw + v * wsmem) + lane;
+                for (int j = 0; j < K; ++j) {
+                    const unsigned long long key = other[j * 32];
+                    if ((int)(unsigned)key >= 0) enter(key);  // no sentinel
+                }
+            }
+        }
+    }
+    if (!live || ((wide >> lane) & 1u)) return;
     for (int n = K - 1; n > 0; --n) {
         const unsigned long long end = heap[n * 32];
         heap[n * 32] = heap[0];
@@ -712,7 +736,14 @@ template <bool BWD, int SEED, int BATCH>
 cudaError_t launch_batch(const Bufs &b, const ScanCall &c)
 {
     const int G = scan_groups(c.n_cand), gs = scan_group_size(c.n_cand);
-    const size_t smem = warp_smem(b.kmax, BATCH, 1 + (BWD ? 1 : 0) + (SEED == kSeedHeap ? 1 : 0));
+    int warps = 1;
+    if (BATCH == kBatchFew && SEED > 0 && !scan_leaves_walks(b, c.n_cand, BWD)) {  // who walks is one warp's choice
+        const long long room = (long long)sm_count_scan() * kWarpsMany / ((long long)b.n_rows * G);
+        const int passes = (b.ldc + kCols - 1) / kCols;
+        warps = (int)(room < kMaxSplit ? room : kMaxSplit);
+        if (warps > passes) warps = passes;
+    }
+    const size_t smem = warps * warp_smem(b.kmax, BATCH, 1 + (BWD ? 1 : 0) + (SEED == kSeedHeap ? 1 : 0));
     const long long blocks = (long long)(c.probe ? kProbeRows : b.n_rows) * G;
     if (smem > (size_t)c.max_smem || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const int walks = scan_leaves_walks(b, c.n_cand, BWD);
@@ -723,7 +754,7 @@ cudaError_t launch_batch(const Bufs &b, const ScanCall &c)
     auto kern = k_scan<BWD, SEED, BATCH>;
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kern<<<(unsigned)blocks, 32, smem, c.stream>>>(b, c.n_cand, G, gs, walks, c.own ? 1 : 0, c.gated ? 1 : 0,
+    kern<<<(unsigned)blocks, 32 * warps, smem, c.stream>>>(b, c.n_cand, G, gs, walks, c.own ? 1 : 0, c.gated ? 1 : 0,
                                                    c.probe ? b.n_rows / kProbeRows : 0);
     return cudaGetLastError();
 }
