@@ -448,7 +448,8 @@ int issue_step(snn_handle *h, int t)
     return SNN_OK;
 }
 
-int issue_reset(snn_handle *h)
+// matrix: also the initial distance matrix (a forward warm start writes D whole).
+int issue_reset(snn_handle *h, bool matrix = true)
 {
     h->fresh = false;
     h->prev_ok = false;
@@ -461,7 +462,8 @@ int issue_reset(snn_handle *h)
         if (int rc = make_pair(h, h->setup_ev)) return rc;
         SNN_CUDA(cudaEventRecord(h->setup_ev.a, h->stream));
     }
-    if (h->desc.backward) {
+    if (!matrix) {
+    } else if (h->desc.backward) {
         SNN_CUDA(snn::launch_full_distance(b, h->cv, h->npf, h->stream));
         SNN_CUDA(snn::launch_row_dmax(b, h->dmax, h->stream));
         h->n_launch += 1;
@@ -471,7 +473,7 @@ int issue_reset(snn_handle *h)
     if (h->setup_timed) SNN_CUDA(cudaEventRecord(h->setup_ev.b, h->stream));
     h->n_launch += 2;
     h->host_step = 0;
-    h->fresh = true;
+    h->fresh = matrix;
     return SNN_OK;
 }
 
@@ -811,15 +813,20 @@ SNN_API int snn_commit_sequence(snn_handle *h, const int *seq, int n)
     }
     SNN_CUDA(cudaSetDevice(h->device));
     reset_timing(h);
+    const int backward = h->desc.backward;
     if (!h->fresh)
-        if (int rc = issue_reset(h)) return rc;
+        if (int rc = issue_reset(h, backward || n == 0)) return rc;
     const Bufs b = h->bufs();
     if (n > 0) h->fresh = false;
-    for (int t = 0; t < n; ++t) {
-        const int it = h->desc.backward ? h->p - 1 - t : t;
-        SNN_CUDA(snn::launch_force(b, seq[t], it, t, h->total_steps, h->desc.backward, h->stream));
-        const bool sd = t + 1 == n && seeds_for_step(h, n);  // the step after the sequence may use seeds
-        SNN_CUDA(snn::launch_commit(b, h->desc.backward, sd ? h->seeds : nullptr, sd ? h->seed_d : nullptr, h->stream));
+    for (int t = 0; t < n; t += snn::kFeatureSeq) {
+        snn::FeatureSeq q;
+        q.n = std::min(n - t, snn::kFeatureSeq);
+        for (int i = 0; i < snn::kFeatureSeq; ++i) q.f[i] = i < q.n ? seq[t + i] : 0;
+        const bool sd = t + q.n == n && seeds_for_step(h, n);  // the step after the sequence may use them
+        SNN_CUDA(snn::launch_force(b, q, t, h->total_steps, backward, h->stream));
+        if (t + q.n == h->total_steps) --q.n;  // nothing is scored after the last step
+        SNN_CUDA(snn::launch_commit_seq(b, q, backward, !backward && t == 0, h->cv, h->npf, sd ? h->seeds : nullptr,
+                                        sd ? h->seed_d : nullptr, h->stream));
         h->seeds_ok = sd;
     }
     h->host_step = n;

@@ -163,6 +163,15 @@ cudaError_t launch_walk(const Bufs &b, cudaStream_t s);
 constexpr int kSeedsPerLane = 8;        // seed columns each lane of the commit keeps: the nearest of each eighth of its columns
 constexpr int kSeeds = 32 * kSeedsPerLane;  // seed columns per row
 cudaError_t launch_commit(const Bufs &b, int backward, int *seeds, float *seed_d, cudaStream_t s);
+// Known features (a warm start), in their order; start: from the empty matrix of
+// a forward selection (D need not hold anything).
+constexpr int kFeatureSeq = 16;
+struct FeatureSeq {
+    int n;
+    int f[kFeatureSeq];
+};
+cudaError_t launch_commit_seq(const Bufs &b, const FeatureSeq &seq, int backward, bool start, int cv, int npf, int *seeds,
+                              float *seed_d, cudaStream_t s);
 
 // First forward step of a holdout problem from per-feature sorted training
 // values (snn_sorted.cu): sort at load, then one thread per problem.
@@ -195,6 +204,7 @@ cudaError_t launch_row_dmax(const Bufs &b, float *dmax, cudaStream_t s);
 cudaError_t launch_feature_variance(const Bufs &b, float *var, float4 *stat, cudaStream_t s);
 // perm[0..p) = features by ascending var (NaN last, ties by id): the candidate slot order.
 cudaError_t launch_feature_order(const float *var, int p, int *perm, cudaStream_t s);
-cudaError_t launch_force(const Bufs &b, int w, int it, int t, int total_steps, int backward, cudaStream_t s);
+// Record the features of seq as the winners of steps t, t + 1, ... without scoring them.
+cudaError_t launch_force(const Bufs &b, const FeatureSeq &seq, int t, int total_steps, int backward, cudaStream_t s);
 
 }  // namespace snn

@@ -308,22 +308,26 @@ __global__ void __launch_bounds__(32) k_select(Bufs b, int n_cand, int it, int t
     if (t + 1 >= total_steps) st->done = 1;
 }
 
-// Warm start: record a given winner without scoring (same bookkeeping as
-// k_select), so the commit kernel and later steps see it.
-__global__ void __launch_bounds__(32) k_force(Bufs b, int w, int it, int t, int total_steps, int backward)
+// Warm start: record given winners without scoring them (same bookkeeping as
+// k_select), so the commit kernel and later steps see them.
+__global__ void __launch_bounds__(32) k_force(Bufs b, FeatureSeq seq, int t0, int total_steps, int backward)
 {
     State *st = b.st;
-    if (st->done) return;
-    next_candidates(b, w, backward);
-    if (threadIdx.x != 0) return;
-    st->winner = w;
-    b.order[it] = w;
-    b.err[it] = 0.0f;
-    b.err64[it] = 0.0;
-    b.stepk[it] = 0;
-    st->num_final = backward ? b.p - (t + 1) : t + 1;
-    st->step = t + 1;
-    if (t + 1 >= total_steps) st->done = 1;
+    for (int i = 0; i < seq.n; ++i) {
+        const int t = t0 + i, it = backward ? b.p - 1 - t : t, w = seq.f[i];
+        next_candidates(b, w, backward);
+        if (threadIdx.x == 0) {
+            st->winner = w;
+            b.order[it] = w;
+            b.err[it] = 0.0f;
+            b.err64[it] = 0.0;
+            b.stepk[it] = 0;
+            st->num_final = backward ? b.p - (t + 1) : t + 1;
+            st->step = t + 1;
+            if (t + 1 >= total_steps) st->done = 1;
+        }
+        __syncwarp();
+    }
 }
 
 __global__ void k_reset_state(Bufs b, int backward, int total_steps)
@@ -496,9 +500,9 @@ cudaError_t launch_select(const Bufs &b, int n_cand, int it, int t, int total_st
     return cudaGetLastError();
 }
 
-cudaError_t launch_force(const Bufs &b, int w, int it, int t, int total_steps, int backward, cudaStream_t s)
+cudaError_t launch_force(const Bufs &b, const FeatureSeq &seq, int t, int total_steps, int backward, cudaStream_t s)
 {
-    k_force<<<1, 32, 0, s>>>(b, w, it, t, total_steps, backward);
+    k_force<<<1, 32, 0, s>>>(b, seq, t, total_steps, backward);
     return cudaGetLastError();
 }
 
