@@ -156,6 +156,7 @@ __global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit, kB
     k_scan(Bufs b, int n_cand, int G, int gs, int walks, int own, int gated, int probe)
 {
     constexpr int kBuf = 2 * kBatch;
+    constexpr bool kHold = !BWD && kBatch == kBatchMany;  // push once per two passes (k = 50 of 50,021 x 24,989: 310 -> 303 ms)
     extern __shared__ __align__(16) unsigned char smraw[];
     if (b.st->done) return;
     if (gated && b.st->full_scan) return;  // the dense scorer takes the step
@@ -216,42 +217,36 @@ __global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit, kB
         float L[SEED];  // ascending; the first SEED - K entries -inf, so the k-th is the last
 #pragma unroll
         for (int j = 0; j < SEED; ++j) L[j] = j < SEED - K ? -INFINITY : INFINITY;
-        const int *seeds = b.seeds + (size_t)r * kSeeds + lane;
-        const float *seed_d = b.seed_d + (size_t)r * kSeeds + lane;
-        int ni = __ldg(seeds);
-        float nd = __ldg(seed_d);
+        const int4 *seeds = reinterpret_cast<const int4 *>(b.seeds + (size_t)r * kSeeds);
+        const float4 *seed_d4 = reinterpret_cast<const float4 *>(b.seed_d + (size_t)r * kSeeds);
+        const float2 xv2 = make_float2(xv, xv);
+        int4 ia = __ldg(seeds), ib = __ldg(seeds + 1);  // -1 for an absent column, its distance +inf
 #pragma unroll 1
-        for (int j0 = 0; j0 < kSeeds; j0 += 32) {
-            const int myi = ni;
-            const float myd = nd;
-            if (j0 + 32 < kSeeds) {
-                ni = __ldg(seeds + j0 + 32);
-                nd = __ldg(seed_d + j0 + 32);
+        for (int j = 0; j < kSeeds / 4; j += 2) {
+            auto at = [&](int i) { return __ldg(xg + (size_t)max(i, 0) * 32); };
+            const float2 x0 = make_float2(at(ia.x), at(ia.y)), x1 = make_float2(at(ia.z), at(ia.w));
+            const float2 x2 = make_float2(at(ib.x), at(ib.y)), x3 = make_float2(at(ib.z), at(ib.w));
+            const float4 da = __ldg(seed_d4 + j), db = __ldg(seed_d4 + j + 1);
+            if (j + 2 < kSeeds / 4) {
+                ia = __ldg(seeds + j + 2);
+                ib = __ldg(seeds + j + 3);
             }
-#pragma unroll 1
-            for (int l0 = 0; l0 < 32; l0 += 8) {
-                float D[8], x[8];
+            auto least = [&](float4 d, float2 xa, float2 xb) {  // a NaN is left out
+                const float2 u = add2(make_float2(d.x, d.y), sq2(sub2(xv2, xa))), v = add2(make_float2(d.z, d.w), sq2(sub2(xv2, xb)));
+                return fminf(fminf(u.x, u.y), fminf(v.x, v.y));
+            };
+            const float va = least(da, x0, x1), vb = least(db, x2, x3);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    D[i] = __shfl_sync(kFull, myd, l0 + i);  // +inf for an absent column (-1)
-                    x[i] = __ldg(xg + (size_t)max(__shfl_sync(kFull, myi, l0 + i), 0) * 32);
-                }
+            for (int i = 0; i < 8; i += P) {
+                const float v = P == 8 ? fminf(va, vb) : i ? vb : va;
+                if (__any_sync(kFull, v < L[SEED - 1])) {
 #pragma unroll
-                for (int i = 0; i < 8; i += P) {
-                    float v = INFINITY;
-#pragma unroll
-                    for (int u = 0; u < P; ++u) {
-                        const float t = __fsub_rn(xv, x[i + u]);
-                        v = fminf(v, __fadd_rn(D[i + u], __fmul_rn(t, t)));  // a NaN is left out
-                    }
-                    if (__any_sync(kFull, v < L[SEED - 1])) {
-#pragma unroll
-                        for (int q = SEED - 1; q > 0; --q) L[q] = fminf(L[q], fmaxf(L[q - 1], v));
-                        L[0] = fminf(L[0], v);
-                    }
+                    for (int q = SEED - 1; q > 0; --q) L[q] = fminf(L[q], fmaxf(L[q - 1], v));
+                    L[0] = fminf(L[0], v);
                 }
             }
         }
+        const float *seed_d = b.seed_d + (size_t)r * kSeeds + lane;
         if (act) lim = fminf(L[SEED - 1], kCap);
         set_near(__ldg(seed_d + 3 * 32), __ldg(seed_d + 4 * 32), __ldg(seed_d + 7 * 32));
     }
@@ -477,14 +472,20 @@ __global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit, kB
         if (probe) return;
     }
     float4 nxt[kUnroll];
-    auto first_columns = [&] {
+    // The next pass' columns.  Past the row any value does: they are masked.
+    auto columns = [&](int q0) {
+        if (q0 + kCols <= b.ldc) {
+            const float4 *at = row + (q0 >> 2) + lane;
 #pragma unroll
-        for (int u = 0; u < kUnroll; ++u) {
-            const int q = w * (kCols / 4) + u * 32 + lane;
-            nxt[u] = q < n4 ? __ldg(row + q) : make_float4(INFINITY, INFINITY, INFINITY, INFINITY);
+            for (int u = 0; u < kUnroll; ++u) nxt[u] = __ldg(at + u * 32);
+        } else {
+#pragma unroll
+            for (int u = 0; u < kUnroll; ++u) nxt[u] = __ldg(row + min((q0 >> 2) + u * 32 + lane, n4 - 1));
         }
     };
-    first_columns();
+    unsigned held = 0u;    // the columns of a pass, pushed together with those of the next
+    bool second = false;
+    columns(w * kCols);
     // kSeedHeap: a pass for the seed columns first
     for (int q0 = SEED == kSeedHeap ? -kCols : w * kCols;; q0 += warps * kCols) {
         const bool last = q0 >= b.ldc;  // no columns left: empty the queues
@@ -504,11 +505,7 @@ __global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit, kB
             };
             m16 = below(!BWD && stage == 0 ? fminf(H, near) : H);
             if (!BWD && stage == 1) m16 &= ~below(near);
-#pragma unroll
-            for (int u = 0; u < kUnroll; ++u) {
-                const int q = (q0 >> 2) + (kUnroll * warps + u) * 32 + lane;
-                nxt[u] = q < n4 ? __ldg(row + q) : make_float4(INFINITY, INFINITY, INFINITY, INFINITY);
-            }
+            columns(q0 + warps * kCols);
             if (q0 + kCols > b.ldc) {  // past the row
 #pragma unroll
                 for (int u = 0; u < kUnroll; ++u)
@@ -523,17 +520,28 @@ __global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit, kB
                 }
             }
         }
-        // Rarely more columns than the queue has room for: then 128 at a time.
-        const int step = __reduce_add_sync(kFull, __popc(m16)) > kQueue - kBatch - 32 ? 4 : 16;
-        for (int part = 0; part < 16; part += step) {
+        if (kHold && !second && !drainall) {
+            held = m16;
+            second = true;
+            continue;
+        }
+        const unsigned m32 = kHold ? held | m16 << 16 : m16;  // bits 0 to 15: the pass before
+        held = 0u;
+        second = false;
+        const int base = kHold ? q0 - warps * kCols : q0;
+        // Rarely more columns than the queue has room for: then a pass, or 128, at a time.
+        const unsigned cnt = __reduce_add_sync(kFull, __popc(m32 & 0xffffu) | __popc(m32 >> 16) << 16);
+        const unsigned room = kQueue - kBatch - 32, c0 = cnt & 0xffffu, c1 = cnt >> 16;
+        const int step = c0 + c1 <= room ? 32 : max(c0, c1) <= room ? 16 : 4;
+        for (int part = 0; part < (kHold ? 32 : 16); part += step) {
             // each lane appends its columns, in no particular order
-            unsigned mp = (m16 >> part) & ((1u << step) - 1u);
+            unsigned mp = (m32 >> part) & (0xffffffffu >> (32 - step));
             for (unsigned any = __ballot_sync(kFull, mp != 0u); any; any = __ballot_sync(kFull, mp != 0u)) {
                 if (mp) {
                     const int i = __ffs(mp) - 1 + part;
                     mp &= mp - 1;
                     const int at = __popc(any & ((1u << lane) - 1u));
-                    const int col = q0 + 128 * (i >> 2) + 4 * lane + (i & 3);
+                    const int col = base + 128 * (i >> 2) + 4 * lane + (i & 3) + (kSplit ? (i >> 4) * (warps - 1) * kCols : 0);
                     if constexpr (BWD) wait[(ah + an + at) & (kQueue - 1)] = col;
                     else queue[(qh + qn + at) & (kQueue - 1)] = col;
                 }
@@ -566,27 +574,38 @@ __global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit, kB
                     // the first queued columns against every candidate of the group
                     const int n = min(qn, kBatch);
                     int col[kBatch];
-                    float d[kBatch], x[kBatch];
+                    float2 d[kBatch / 2], x[kBatch / 2];
 #pragma unroll
-                    for (int i = 0; i < kBatch; ++i) {
-                        col[i] = i < n ? queue[(qh + i) & (kQueue - 1)] : 0;
-                        d[i] = __ldg(Dr + col[i]);
-                        x[i] = __ldg(xg + (size_t)col[i] * 32);
+                    for (int i = 0; i < kBatch; i += 4) {  // qh is a multiple of 4
+                        const int4 v = *reinterpret_cast<const int4 *>(queue + ((qh + i) & (kQueue - 1)));
+                        col[i] = v.x;
+                        col[i + 1] = v.y;
+                        col[i + 2] = v.z;
+                        col[i + 3] = v.w;
                     }
-                    qh = (qh + n) & (kQueue - 1);
+                    if (n < kBatch) {
+#pragma unroll
+                        for (int i = 0; i < kBatch; ++i) col[i] = i < n ? col[i] : 0;
+                    }
+#pragma unroll
+                    for (int i = 0; i < kBatch; i += 2) {
+                        d[i / 2] = make_float2(__ldg(Dr + col[i]), __ldg(Dr + col[i + 1]));
+                        x[i / 2] = make_float2(__ldg(xg + (size_t)col[i] * 32), __ldg(xg + (size_t)col[i + 1] * 32));
+                    }
                     qn -= n;
+                    qh = qn ? (qh + n) & (kQueue - 1) : 0;
                     unsigned pm = 0u;
 #pragma unroll
-                    for (int i = 0; i < kBatch; ++i) {
-                        const float t = __fsub_rn(xv, x[i]);
-                        const float s = __fmul_rn(t, t);
-                        d[i] = BWD ? __fsub_rn(d[i], s) : __fadd_rn(d[i], s);
-                        pm |= d[i] <= lim && i < n ? 1u << i : 0u;
+                    for (int i = 0; i < kBatch; i += 2) {
+                        const float2 s = sq2(sub2(make_float2(xv, xv), x[i / 2]));
+                        d[i / 2] = BWD ? sub2(d[i / 2], s) : add2(d[i / 2], s);
+                        pm |= (d[i / 2].x <= lim ? 1u << i : 0u) | (d[i / 2].y <= lim ? 2u << i : 0u);
                     }
+                    pm &= (1u << n) - 1u;
                     if (__any_sync(kFull, pm != 0u)) {
 #pragma unroll
                         for (int i = 0; i < kBatch; ++i)
-                            if ((pm >> i) & 1u) buf[32 * nb++] = pack_key<BWD>(d[i], col[i]);
+                            if ((pm >> i) & 1u) buf[32 * nb++] = pack_key<BWD>(i & 1 ? d[i / 2].y : d[i / 2].x, col[i]);
                     }
                     if (__any_sync(kFull, nb > kBuf - kBatch)) flush();
                 }
@@ -617,7 +636,7 @@ __global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit, kB
             stage = 1;
             nseed = noseed;
             q0 = (w - warps) * kCols;
-            first_columns();
+            columns(w * kCols);
         }
     }
 
