@@ -109,6 +109,11 @@ struct snn_handle {
     int bwd_dense = 0;            // backward: 1 the dense scorer is faster on the loaded data, -1 not known (probe each step)
     int *walk = nullptr, *n_walk = nullptr;  // forward holdout: problems left to k_walk, and how many
     bool sorted_start = true;     // SNN_OPT_SORTED_START
+    int2 *near_list = nullptr;  // forward, many columns: the commit's near columns per row
+    float4 *near_info = nullptr, *near_next = nullptr;
+    bool no_list = false;         // there was no memory for them
+    bool near_ok = false;         // near_next is the last commit's
+    bool list_ok = false;         // near_list holds the current D's near columns
     bool seeds_ok = false;        // seeds hold the current D's seed columns
     int seed_step = 0;            // SNN_OPT_SEED_STEP: first forward step scored from seed bounds; 0: first_seeded
     unsigned long long *fcount = nullptr;  // filter counters of the TMA-fed scorer (3)
@@ -187,6 +192,9 @@ struct snn_handle {
         b.n_walk = n_walk;
         b.sval = sval;
         b.sidx = sidx;
+        b.near_list = nullptr;
+        b.near_info = near_info;
+        b.near_next = near_next;
         b.only_if_full = 0;
         return b;
     }
@@ -383,6 +391,7 @@ int issue_step(snn_handle *h, int t)
         // open (30,000 x 15,000 x 40 such features, second step: 23.7 ms, dense 8.3);
         // the probe and the launch that returns at once take 0.1 ms of a fwd-64k step.
         const bool gated = (backward ? h->bwd_dense < 0 : t <= 3) && snn::scan_worth_probing(b, n_cand);
+        if (h->list_ok && seeding == snn::kGivenSeeds) b.near_list = h->near_list;
         if (gated) SNN_CUDA(snn::launch_scan_probe(b, n_cand, backward, seeding, h->max_smem, h->stream));
         SNN_CUDA(snn::launch_scan(b, n_cand, backward, seeding, gated, h->max_smem, h->stream));
         if (snn::scan_leaves_walks(b, n_cand, backward)) {
@@ -437,7 +446,10 @@ int issue_step(snn_handle *h, int t)
             SNN_CUDA(cudaEventRecord(ce->a, h->stream));
         }
         const bool sd = seeds_for_step(h, t + 1);
-        SNN_CUDA(snn::launch_commit(b, backward, sd ? h->seeds : nullptr, sd ? h->seed_d : nullptr, h->stream));
+        h->list_ok = sd && h->near_list && h->near_ok;
+        h->near_ok = sd && h->near_list;
+        b.near_list = h->near_list;
+        SNN_CUDA(snn::launch_commit(b, backward, sd ? h->seeds : nullptr, sd ? h->seed_d : nullptr, h->list_ok, h->stream));
         h->seeds_ok = sd;
         if (ce) {
             SNN_CUDA(cudaEventRecord(ce->b, h->stream));
@@ -454,6 +466,7 @@ int issue_reset(snn_handle *h, bool matrix = true)
     h->fresh = false;
     h->prev_ok = false;
     h->seeds_ok = false;
+    h->near_ok = h->list_ok = false;
     h->last_ncand = 0;
     const Bufs b = h->bufs();
     SNN_CUDA(snn::launch_reset_state(b, h->desc.backward, h->total_steps, h->stream));
@@ -523,6 +536,10 @@ static int validate_desc(const snn_desc *d, int *kmax_out)
     return SNN_OK;
 }
 
+// Forward problems of that many training columns keep their near columns (16 KB
+// per row): below, the scan's passes over the row are few.
+constexpr int kNearListCols = 16384;
+
 // Device bytes a handle for this descriptor allocates (buffers of snn_create
 // plus the load staging buffer), for the batch's memory waves.
 static size_t handle_bytes(const snn_desc *d, int kmax)
@@ -532,7 +549,8 @@ static size_t handle_bytes(const snn_desc *d, int kmax)
     const size_t n_rows = cv ? n_cols : (size_t)d->n_val;
     const size_t ldc = (size_t)round_up(d->n_train, snn::kPadCols);
     const size_t ldr = cv ? ldc : (size_t)round_up((int)n_rows, snn::kPadCols);
-    const size_t M = d->backward ? 0 : 2 * (size_t)snn::kSeeds + p;  // seed columns, distances, bounds
+    const size_t M = d->backward ? 0 : 2 * (size_t)snn::kSeeds + p +  // seed columns, distances, bounds, near columns
+                                           (d->n_train >= kNearListCols ? 2 * (size_t)snn::kNearList + 8 : 0);
     (void)kmax;
     size_t f = p * ldc + n_rows * ldc + p * (size_t)d->num_k_vals * n_rows + std::max(n_rows, n_cols) * p +
                n_rows * M + n_cols + n_rows;
@@ -583,6 +601,11 @@ static int carve_buffers(snn_handle *h, Arena &a)
         if ((rc = carve(a, &h->seeds, (size_t)h->n_rows * snn::kSeeds, "seed columns"))) return rc;
         if ((rc = carve(a, &h->seed_d, (size_t)h->n_rows * snn::kSeeds, "seed distances"))) return rc;
         if ((rc = carve(a, &h->sbound, p * h->n_rows, "seed bounds"))) return rc;
+        if (h->n_cols >= kNearListCols && !h->no_list) {
+            if ((rc = carve(a, &h->near_list, (size_t)h->n_rows * snn::kNearList, "near columns"))) return rc;
+            if ((rc = carve(a, &h->near_info, (size_t)h->n_rows, "near columns"))) return rc;
+            if ((rc = carve(a, &h->near_next, (size_t)h->n_rows, "near columns"))) return rc;
+        }
     }
     const size_t groups = (p + 31) / 32;
     if ((rc = carve(a, &h->xg, groups * h->ldc * 32, "packed candidates"))) return rc;
@@ -654,7 +677,15 @@ SNN_API int snn_create(const snn_desc *d, snn_handle **out)
     if (h->plan.cc == 0)
         return bail(fail(SNN_ERR_UNSUPPORTED, "k_max=%d is above the supported maximum of %d", kmax, snn::kScoreMaxK));
     if (!h->desc.backward && !cv) h->stemp_bytes = snn::sort_temp_bytes(h->p, h->ldc);
-    if ((rc = take_buffers(h, h->block, "a problem", [&](Arena &a) { return carve_buffers(h, a); }))) return bail(rc);
+    rc = take_buffers(h, h->block, "a problem", [&](Arena &a) { return carve_buffers(h, a); });
+    if (rc == SNN_ERR_NOMEM && h->near_list) {  // the scan does without them
+        h->near_list = nullptr;
+        h->near_info = h->near_next = nullptr;
+        h->no_list = true;
+        cudaGetLastError();
+        rc = take_buffers(h, h->block, "a problem", [&](Arena &a) { return carve_buffers(h, a); });
+    }
+    if (rc) return bail(rc);
     h->stream = h->block.stream;
     if (!h->stream && cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess)
         return bail(fail(SNN_ERR_CUDA, "cudaStreamCreate failed"));
@@ -828,6 +859,7 @@ SNN_API int snn_commit_sequence(snn_handle *h, const int *seq, int n)
         SNN_CUDA(snn::launch_commit_seq(b, q, backward, !backward && t == 0, h->cv, h->npf, sd ? h->seeds : nullptr,
                                         sd ? h->seed_d : nullptr, h->stream));
         h->seeds_ok = sd;
+        h->near_ok = h->list_ok = false;
     }
     h->host_step = n;
     SNN_CUDA(cudaStreamSynchronize(h->stream));
@@ -1070,12 +1102,14 @@ SNN_API int snn_set_option(snn_handle *h, int option, int value)
             return fail(SNN_ERR_UNSUPPORTED, "the TMA-fed kernel handles k_max <= 64");
         h->kernel = value;
         h->seeds_ok = false;
+        h->near_ok = h->list_ok = false;
         return SNN_OK;
     case SNN_OPT_SORTED_START: h->sorted_start = value != 0; return SNN_OK;
     case SNN_OPT_SEED_STEP:
         if (value < 1) return fail(SNN_ERR_ARG, "seed step %d must be >= 1", value);
         h->seed_step = value;
         h->seeds_ok = false;
+        h->near_ok = h->list_ok = false;
         return SNN_OK;
     case SNN_OPT_COUNTERS: h->count_filter = value != 0; return SNN_OK;
     default: return fail(SNN_ERR_ARG, "unknown option %d", option);

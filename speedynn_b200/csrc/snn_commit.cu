@@ -60,11 +60,30 @@ __device__ __forceinline__ void store_seeds(float (&sv)[kSeedsPerLane], int (&si
     }
 }
 
+// The middle and the largest of the lanes' sorted seeds, averaged: about the
+// row's 172nd and 680th smallest distance; their power law goes on to the
+// 1,024th (snn_scan.cu).  From these, what the next commit lists by: that
+// distance, grown by 1.1 times what the last feature added (`last`: the same of
+// the commit before).  On the fwd-64k and fwd-200k data 480 to 1,500 columns lie
+// below it from the fifth step on, more than kNearList for 1 to 3 % of the rows.
+__device__ __forceinline__ float4 near_of(const float (&sv)[kSeedsPerLane], float last)
+{
+    float mid = 0.5f * (sv[3] + sv[4]), far = sv[kSeedsPerLane - 1];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        mid += __shfl_xor_sync(0xffffffffu, mid, o);
+        far += __shfl_xor_sync(0xffffffffu, far, o);
+    }
+    const float near = far * 0.03125f * powf(far / mid, 0.298f);  // ln(1024 / 680) / ln(680 / 172)
+    const float grow = last > 0.0f && last < near ? 1.0f + 1.1f * (near - last) / near : 1.5f;
+    return make_float4(near, near * grow, mid * 0.03125f * grow, 0.0f);
+}
+
 // Three blocks of 256 threads per SM, each lane with four float4 loads of D in
 // flight: the stream needs that many bytes in flight to stay HBM-bound (four
 // blocks with two loads per lane while the seed lists take registers: 44.0
 // against 43.0 ms of commits per fwd-64k selection).
-template <bool BWD, bool SEEDS>
+template <bool BWD, bool SEEDS, bool LIST>
 __global__ void __launch_bounds__(256, 3) k_commit(Bufs b, int *seeds, float *seed_d)
 {
     if (b.st->done) return;
@@ -87,6 +106,13 @@ __global__ void __launch_bounds__(256, 3) k_commit(Bufs b, int *seeds, float *se
         for (int j = 0; j < kSeedsPerLane; ++j) {
             sv[j] = INFINITY;
             si[j] = -1;
+        }
+        float4 by;
+        int found = 0;  // columns below by.y
+        int2 *list = nullptr;
+        if (LIST) {
+            by = b.near_next[r];
+            list = b.near_list + (size_t)r * kNearList;
         }
 #pragma unroll
         for (int h = 0; h < H; ++h) {
@@ -129,6 +155,23 @@ __global__ void __launch_bounds__(256, 3) k_commit(Bufs b, int *seeds, float *se
                         }
                     }
                 }
+                if (LIST) {
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const int q = q0 + u * 32 + lane;
+                        const float v[4] = {d[u].x, d[u].y, d[u].z, d[u].w};
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const bool in = q < end && v[e] < by.y;
+                            const unsigned m = __ballot_sync(0xffffffffu, in);
+                            if (m) {
+                                const int at = found + __popc(m & ((1u << lane) - 1u));
+                                if (in && at < kNearList) list[at] = make_int2(4 * q + e, __float_as_int(v[e]));
+                                found += __popc(m);
+                            }
+                        }
+                    }
+                }
             }
         }
         if (SEEDS) {
@@ -136,6 +179,13 @@ __global__ void __launch_bounds__(256, 3) k_commit(Bufs b, int *seeds, float *se
 #pragma unroll
             for (int j = 0; j < kSeedsPerLane; ++j) si[j] = si[j] < 0 ? -1 : 4 * si[j] + (j & 3);
             store_seeds(sv, si, seeds, seed_d, r, lane);
+            if (b.near_next) {
+                const float4 next = near_of(sv, LIST ? by.x : 0.0f);
+                if (lane == 0) {
+                    b.near_next[r] = next;
+                    if (LIST) b.near_info[r] = make_float4(by.y < FLT_MAX ? (float)found : INFINITY, by.y, by.z, 0.0f);
+                }
+            }
         }
     }
 }
@@ -267,14 +317,15 @@ int sm_count_commit()
 
 }  // namespace
 
-cudaError_t launch_commit(const Bufs &b, int backward, int *seeds, float *seed_d, cudaStream_t s)
+cudaError_t launch_commit(const Bufs &b, int backward, int *seeds, float *seed_d, bool list, cudaStream_t s)
 {
     int grid = (b.n_rows + 7) / 8;
     const int cap = sm_count_commit() * 6;
     if (grid > cap) grid = cap;
-    if (backward) k_commit<true, false><<<grid, 256, 0, s>>>(b, nullptr, nullptr);
-    else if (seeds && seed_d) k_commit<false, true><<<grid, 256, 0, s>>>(b, seeds, seed_d);
-    else k_commit<false, false><<<grid, 256, 0, s>>>(b, nullptr, nullptr);
+    if (backward) k_commit<true, false, false><<<grid, 256, 0, s>>>(b, nullptr, nullptr);
+    else if (seeds && seed_d && list) k_commit<false, true, true><<<grid, 256, 0, s>>>(b, seeds, seed_d);
+    else if (seeds && seed_d) k_commit<false, true, false><<<grid, 256, 0, s>>>(b, seeds, seed_d);
+    else k_commit<false, false, false><<<grid, 256, 0, s>>>(b, nullptr, nullptr);
     return cudaGetLastError();
 }
 

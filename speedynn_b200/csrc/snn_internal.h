@@ -111,6 +111,13 @@ struct Bufs {
     int *n_walk;
     const float *sval;
     const int *sidx;
+    // forward: each row's near columns as the last commit found them (null: none
+    // kept): (column, distance) [n_rows][kNearList], all columns below near_info's y
+    // if its x, their number, is at most kNearList; z: a distance below which about
+    // a quarter of them lie; and what the next commit lists by (k_commit)
+    int2 *near_list;
+    float4 *near_info;
+    float4 *near_next;
     int only_if_full;  // scoring kernels return at once unless st->full_scan is set
 };
 
@@ -162,7 +169,9 @@ cudaError_t launch_walk(const Bufs &b, cudaStream_t s);
 // buffers also keep kSeeds near columns per row for the next step's bounds.
 constexpr int kSeedsPerLane = 8;        // seed columns each lane of the commit keeps: the nearest of each eighth of its columns
 constexpr int kSeeds = 32 * kSeedsPerLane;  // seed columns per row
-cudaError_t launch_commit(const Bufs &b, int backward, int *seeds, float *seed_d, cudaStream_t s);
+// list: write b.near_list by the last such commit's b.near_next.
+constexpr int kNearList = 2048;
+cudaError_t launch_commit(const Bufs &b, int backward, int *seeds, float *seed_d, bool list, cudaStream_t s);
 // Known features (a warm start), in their order; start: from the empty matrix of
 // a forward selection (D need not hold anything).
 constexpr int kFeatureSeq = 16;

@@ -76,6 +76,7 @@ constexpr float kQueueCost = 14.0f, kWalkStart = 3000.0f, kWalkCost = 8.0f, kPas
 // per candidate (measured: 30,000 x 15,000 x 38 8 ms, the scan 14 with 68 % open).
 constexpr float kReadCost = 0.25f, kTestCost = 4.0f, kDenseCost = 0.28f;
 constexpr int kProbeRows = 64;
+constexpr int kNearLeast = 256;  // of fewer near columns nothing is gained: the row is read for its others
 static_assert(kSeedsPerLane == 8, "the commit and the scan keep eight seeds per lane");
 static_assert(kQueue >= kSeeds && kQueue >= 128 + 16 + 32, "room for a pass's columns");
 
@@ -144,7 +145,7 @@ constexpr int kSeedNone = 0, kSeedHeap = -1;
 // loads of one batch under the work of the last one at 16 warps 139.6);
 // problems of at most one such wave of warps, whose time is the chain of
 // gathers of one warp, take batches of 16.
-constexpr int kBatchMany = 4, kBatchFew = 16, kWarpsMany = 28;
+constexpr int kBatchMany = 4, kBatchFew = 16, kWarpsMany = 28, kWarpsHeap = 24;
 // ... and, forward from given bounds, two warps for each (row, group), each with
 // every other pass over the row; the first one merges the lists (steps 3 to 8 of
 // 2,000 x 1,000 x 20: 0.50 -> 0.39 ms; four warps 0.45; backward, where the work
@@ -152,7 +153,8 @@ constexpr int kBatchMany = 4, kBatchFew = 16, kWarpsMany = 28;
 constexpr int kMaxSplit = 2;
 
 template <bool BWD, int SEED, int kBatch>
-__global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit, kBatch == kBatchMany ? kWarpsMany : 16 / kMaxSplit)
+__global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit,
+                                  kBatch != kBatchMany ? 16 / kMaxSplit : SEED == kSeedHeap ? kWarpsHeap : kWarpsMany)
     k_scan(Bufs b, int n_cand, int G, int gs, int walks, int own, int gated, int probe)
 {
     constexpr int kBuf = 2 * kBatch;
@@ -173,6 +175,7 @@ __global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit, kB
     int *queue = reinterpret_cast<int *>(smraw + w * wsmem + lists_at);
     int *wait = queue + kQueue;                  // backward: columns before the second test
     int *own_seed = queue + (BWD ? 2 : 1) * kQueue;  // kSeedHeap: the lanes' seed columns
+    float *queue_d = reinterpret_cast<float *>(queue + kQueue);  // near columns: the queued columns' distances (own_seed's place)
 
     const int slot = g * gs + lane;
     const bool live = lane < gs && slot < n_cand;
@@ -203,6 +206,21 @@ __global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit, kB
         const float v = d8 * 0.03125f * powf(d8 / mid, 0.298f);  // ln(1024 / 680) / ln(680 / 172)
         if (v < FLT_MAX) near = v;  // otherwise (a lane without eight seeds, ties at 0): one stage for all columns
     };
+
+    // The row's near columns, where the commit could list them all.
+    constexpr bool kLists = !BWD && (SEED > 0 || SEED == kSeedHeap);
+    bool listed = false;  // taking them now
+    int n_near = 0;
+    float quarter = 0.0f;
+    if (kLists && b.near_list && !probe) {
+        const float4 info = __ldg(b.near_info + r);
+        listed = info.x <= (float)kNearList && info.x >= (float)kNearLeast && warps == 1;
+        if (listed) {
+            n_near = (int)info.x;
+            near = info.y;
+            quarter = info.z;
+        }
+    }
 
     // lim: distances above it cannot enter the lane's list.
     float lim = act ? kCap : -INFINITY;
@@ -248,7 +266,7 @@ __global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit, kB
         }
         const float *seed_d = b.seed_d + (size_t)r * kSeeds + lane;
         if (act) lim = fminf(L[SEED - 1], kCap);
-        set_near(__ldg(seed_d + 3 * 32), __ldg(seed_d + 4 * 32), __ldg(seed_d + 7 * 32));
+        if (!listed) set_near(__ldg(seed_d + 3 * 32), __ldg(seed_d + 4 * 32), __ldg(seed_d + 7 * 32));
     }
 
     // The list starts as K sentinels at the (inclusive) bound, ordered after every
@@ -270,9 +288,10 @@ __global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit, kB
     // kSeedHeap: the seed columns go through the queue before the row's others; the
     // lane keeps its own (the commit and this kernel give each lane the same
     // columns), ascending, to leave them out afterwards.
+    // (Not with near columns: those make the start.)
     int nseed = 0;  // the lane's seed columns already passed, the next at own_seed[32 * nseed + lane]
-    int noseed = 0;  // entries of own_seed without a column
-    if constexpr (SEED == kSeedHeap) {
+    int noseed = listed ? kSeedsPerLane : 0;  // entries of own_seed without a column
+    if (SEED == kSeedHeap && !listed) {
         int si[kSeedsPerLane];
         if (!own) {
             const float *seed_d = b.seed_d + (size_t)r * kSeeds + lane;
@@ -462,6 +481,7 @@ __global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit, kB
     // first, which leaves nearly exact bounds for the split and for the others
     // (or none of them open).
     int stage = BWD || !(H > near) ? 2 : 0;  // 0: D < near, 1: the rest, 2: all in one
+    bool close = SEED == kSeedHeap && listed;  // first only the nearest quarter of the near columns
     if constexpr (SEED != kSeedHeap) {
         if constexpr (BWD) {
             if (probe) probe_backward();
@@ -485,13 +505,34 @@ __global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit, kB
     };
     unsigned held = 0u;    // the columns of a pass, pushed together with those of the next
     bool second = false;
-    columns(w * kCols);
+    // Near columns, four of 128 per lane and pass: nxt holds this pass' and the next's.
+    const float4 *near4 = reinterpret_cast<const float4 *>(b.near_list + (size_t)r * kNearList) + 2 * lane;
+    auto near_columns = [&](int q) {
+        if (q + 4 * lane < n_near) {
+            nxt[2] = __ldg(near4 + (q >> 1));
+            nxt[3] = __ldg(near4 + (q >> 1) + 1);
+        }
+    };
+    if (listed) {
+        near_columns(0);
+        nxt[0] = nxt[2];
+        nxt[1] = nxt[3];
+        near_columns(128);
+    } else {
+        columns(w * kCols);
+    }
     // kSeedHeap: a pass for the seed columns first
-    for (int q0 = SEED == kSeedHeap ? -kCols : w * kCols;; q0 += warps * kCols) {
-        const bool last = q0 >= b.ldc;  // no columns left: empty the queues
+    for (int q0 = SEED == kSeedHeap && !listed ? -kCols : w * kCols;; q0 += listed ? 128 : warps * kCols) {
+        const bool last = q0 >= (listed ? n_near : b.ldc);  // no columns left: empty the queues
         const bool drainall = last || q0 < 0;
         unsigned m16 = 0u;  // bit 4u + e: this lane's column q0 + 128 u + 4 lane + e has D < H
-        if (SEED != kSeedHeap || q0 >= 0) {
+        if (listed) {  // bit e: this lane's column e
+            const float lo = close ? 0.0f : SEED == kSeedHeap ? quarter : 0.0f, hi = close ? fminf(quarter, H) : H;
+            auto open = [&](float d) { return d < hi && d >= lo; };
+            m16 = (open(nxt[0].y) ? 1u : 0u) | (open(nxt[0].w) ? 2u : 0u) | (open(nxt[1].y) ? 4u : 0u) | (open(nxt[1].w) ? 8u : 0u);
+            const int left = n_near - q0 - 4 * lane;
+            if (left < 4) m16 &= left > 0 ? (1u << left) - 1u : 0u;
+        } else if (SEED != kSeedHeap || q0 >= 0) {
             // the sign of D - H, first column lowest
             auto below = [&](float limit) {
                 const float2 nl = make_float2(-limit, -limit);
@@ -520,15 +561,15 @@ __global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit, kB
                 }
             }
         }
-        if (kHold && !second && !drainall) {
+        if (kHold && !second && !drainall && !listed) {
             held = m16;
             second = true;
             continue;
         }
-        const unsigned m32 = kHold ? held | m16 << 16 : m16;  // bits 0 to 15: the pass before
+        const unsigned m32 = kHold && !listed ? held | m16 << 16 : m16;  // bits 0 to 15: the pass before
         held = 0u;
         second = false;
-        const int base = kHold ? q0 - warps * kCols : q0;
+        const int base = kHold && !listed ? q0 - warps * kCols : q0;
         // Rarely more columns than the queue has room for: then a pass, or 128, at a time.
         const unsigned cnt = __reduce_add_sync(kFull, __popc(m32 & 0xffffu) | __popc(m32 >> 16) << 16);
         const unsigned room = kQueue - kBatch - 32, c0 = cnt & 0xffffu, c1 = cnt >> 16;
@@ -541,9 +582,16 @@ __global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit, kB
                     const int i = __ffs(mp) - 1 + part;
                     mp &= mp - 1;
                     const int at = __popc(any & ((1u << lane) - 1u));
-                    const int col = base + 128 * (i >> 2) + 4 * lane + (i & 3) + (kSplit ? (i >> 4) * (warps - 1) * kCols : 0);
+                    int col = base + 128 * (i >> 2) + 4 * lane + (i & 3) + (kSplit ? (i >> 4) * (warps - 1) * kCols : 0);
                     if constexpr (BWD) wait[(ah + an + at) & (kQueue - 1)] = col;
-                    else queue[(qh + qn + at) & (kQueue - 1)] = col;
+                    else {
+                        if (kLists && listed) {
+                            const float4 v = i & 2 ? nxt[1] : nxt[0];
+                            col = __float_as_int(i & 1 ? v.z : v.x);
+                            queue_d[(qh + qn + at) & (kQueue - 1)] = i & 1 ? v.w : v.y;
+                        }
+                        queue[(qh + qn + at) & (kQueue - 1)] = col;
+                    }
                 }
                 if constexpr (BWD) an += __popc(any);
                 else qn += __popc(any);
@@ -589,7 +637,8 @@ __global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit, kB
                     }
 #pragma unroll
                     for (int i = 0; i < kBatch; i += 2) {
-                        d[i / 2] = make_float2(__ldg(Dr + col[i]), __ldg(Dr + col[i + 1]));
+                        if (kLists && listed) d[i / 2] = *reinterpret_cast<const float2 *>(queue_d + ((qh + i) & (kQueue - 1)));
+                        else d[i / 2] = make_float2(__ldg(Dr + col[i]), __ldg(Dr + col[i + 1]));
                         x[i / 2] = make_float2(__ldg(xg + (size_t)col[i] * 32), __ldg(xg + (size_t)col[i + 1] * 32));
                     }
                     qn -= n;
@@ -625,7 +674,22 @@ __global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit, kB
             }
             if (probe) return;
         }
+        if (kLists && listed && !last) {
+            nxt[0] = nxt[2];
+            nxt[1] = nxt[3];
+            near_columns(q0 + 256);
+        }
         if (last) {
+            if (SEED == kSeedHeap && close) {
+                close = false;
+                flush();
+                near_columns(0);
+                nxt[0] = nxt[2];
+                nxt[1] = nxt[3];
+                near_columns(128);
+                q0 = -128;
+                continue;
+            }
             if (BWD || stage != 0) break;
             flush();
             if (walks) {
@@ -634,6 +698,7 @@ __global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit, kB
             }
             if (!(H > near)) break;
             stage = 1;
+            listed = false;
             nseed = noseed;
             q0 = (w - warps) * kCols;
             columns(w * kCols);
@@ -762,7 +827,7 @@ cudaError_t launch_batch(const Bufs &b, const ScanCall &c)
         warps = (int)(room < kMaxSplit ? room : kMaxSplit);
         if (warps > passes) warps = passes;
     }
-    const size_t smem = warps * warp_smem(b.kmax, BATCH, 1 + (BWD ? 1 : 0) + (SEED == kSeedHeap ? 1 : 0));
+    const size_t smem = warps * warp_smem(b.kmax, BATCH, 1 + (BWD ? 1 : 0) + (SEED == kSeedHeap || (SEED > 0 && b.near_list) ? 1 : 0));
     const long long blocks = (long long)(c.probe ? kProbeRows : b.n_rows) * G;
     if (smem > (size_t)c.max_smem || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const int walks = scan_leaves_walks(b, c.n_cand, BWD);
