@@ -64,9 +64,13 @@ __device__ __forceinline__ void store_seeds(float (&sv)[kSeedsPerLane], int (&si
 // row's 172nd and 680th smallest distance; their power law goes on to the
 // 1,024th (snn_scan.cu).  From these, what the next commit lists by: that
 // distance, grown by 1.1 times what the last feature added (`last`: the same of
-// the commit before).  On the fwd-64k and fwd-200k data 480 to 1,500 columns lie
-// below it from the fifth step on, more than kNearList for 1 to 3 % of the rows.
-__device__ __forceinline__ float4 near_of(const float (&sv)[kSeedsPerLane], float last)
+// the commit before).  The first features change the dimension most: on normal
+// data the n-th part of the columns reaches about n times as far under two
+// features as under one, and 4.5 times as far under three as under two (the
+// median rows of fwd-64k and fwd-200k 72 and 50 for n of 64 and 49, then 5.1 and
+// 4.4).  On those data 70 to 99 % of the lists hold 256 to kNearList columns,
+// except after the fifth feature of fwd-200k (40 %).
+__device__ __forceinline__ float4 near_of(const float (&sv)[kSeedsPerLane], float last, int n_cols)
 {
     float mid = 0.5f * (sv[3] + sv[4]), far = sv[kSeedsPerLane - 1];
 #pragma unroll
@@ -75,7 +79,9 @@ __device__ __forceinline__ float4 near_of(const float (&sv)[kSeedsPerLane], floa
         far += __shfl_xor_sync(0xffffffffu, far, o);
     }
     const float near = far * 0.03125f * powf(far / mid, 0.298f);  // ln(1024 / 680) / ln(680 / 172)
-    const float grow = last > 0.0f && last < near ? 1.0f + 1.1f * (near - last) / near : 1.5f;
+    const float grow = !(last > 0.0f)         ? (float)n_cols * (1.0f / 800.0f)
+                       : near > 8.0f * last ? 4.5f
+                                            : 1.0f + 1.1f * fmaxf(near - last, 0.0f) / near;
     return make_float4(near, near * grow, mid * 0.03125f * grow, 0.0f);
 }
 
@@ -180,7 +186,7 @@ __global__ void __launch_bounds__(256, 3) k_commit(Bufs b, int *seeds, float *se
             for (int j = 0; j < kSeedsPerLane; ++j) si[j] = si[j] < 0 ? -1 : 4 * si[j] + (j & 3);
             store_seeds(sv, si, seeds, seed_d, r, lane);
             if (b.near_next) {
-                const float4 next = near_of(sv, LIST ? by.x : 0.0f);
+                const float4 next = near_of(sv, LIST ? by.x : 0.0f, b.n_cols);
                 if (lane == 0) {
                     b.near_next[r] = next;
                     if (LIST) b.near_info[r] = make_float4(by.y < FLT_MAX ? (float)found : INFINITY, by.y, by.z, 0.0f);
