@@ -91,15 +91,18 @@ def job_value(evals_per_rank, ms_max, world):
 
 
 def scoring_kernel(kmax, option=0):
-    """Name of the scoring kernel the library picks (option 0 = automatic)."""
-    if option == 3 or (option == 0 and kmax <= 64):
-        return "k_score_tma"
-    return "k_score"
+    """Name of the scoring kernel the library picks (option 0 = automatic: the
+    pruned scan, beside the sorted first steps of a forward holdout run)."""
+    if option == 0:
+        return "k_scan"
+    return "k_score_tma" if option == 3 and kmax <= 64 else "k_score"
 
 
-# FP32-pipe operations per evaluation in the roofline's work count: sub, mul,
-# add and compare (the reference's scalar loop); the scorer's filter issues one
-# packed sub and one packed FMA per evaluation plus a sign-bit OR.
+# FP32-pipe operations per evaluation of an exhaustive scorer: sub, mul, add and
+# compare (the reference's scalar loop).  The pruned scan proves from exact bounds
+# that most evaluations cannot enter a list and does not form them, so against
+# this count it runs above the FP32 pipe's peak; what it cannot do without is one
+# read of D per step.
 OPS_PER_EVAL = 4
 
 
@@ -473,7 +476,7 @@ def run_ours(args, world, rank, local):
     e2e_s = allmax((time.perf_counter() - e0) / args.steps, world)
     sel.close()
 
-    # roofline of the scoring kernel: FP32 pipe (OPS_PER_EVAL ops per evaluation) vs one D read
+    # roofline of the scoring kernel: one D read; beside it the FP32 pipe at OPS_PER_EVAL ops per evaluation
     peaks = {}
     try:
         peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
@@ -490,8 +493,8 @@ def run_ours(args, world, rank, local):
     bytes_per_launch = 4.0 * n_val * n_train
     achieved_hbm = bytes_per_launch / avg_score_s * 1e-9
     # the same over the steps that scan every column (forward holdout steps 1
-    # and 2 take their lists from sorted feature values instead, for k <= 64)
-    first_scan = 0 if backward else (2 if k <= 64 else 1)
+    # and, of up to 4,096 columns, 2 take their lists from sorted feature values)
+    first_scan = 0 if backward else (2 if k <= 32 and n_train <= 4096 else 1)
     scan_evals = sum(float(n_val) * n_train * (p - t) for t in range(first_scan, steps))
     scan_s = float(step_score[first_scan:].sum()) / args.steps / 1000.0
     achieved_scan = OPS_PER_EVAL * scan_evals / scan_s * 1e-12 if scan_s > 0 else None
@@ -512,34 +515,26 @@ def run_ours(args, world, rank, local):
             "filter": {"row_chunks": fc["row_chunks"],
                        "flagged_frac": fc["flagged"] / fc["row_chunks"] if fc["row_chunks"] else None,
                        "passing_frac": fc["passed"] / fc["row_chunks"] if fc["row_chunks"] else None,
-                       "note": "(row, 64-column chunk) pairs of the TMA-fed scorer's full passes in one selection "
-                               "(counted in an extra untimed run); flagged = re-scored exactly, passing = held a "
+                       "note": "(row, 64-column chunk) pairs of the dense TMA-fed scorer's full passes in one selection "
+                               "(counted in an extra untimed run, which that scorer takes); flagged = re-scored exactly, passing = held a "
                                "list update candidate"},
-            "roofline": {"bound": "fp32", "kernel": scoring_kernel(k, args.kernel), "achieved": achieved_fp32,
-                         "peak": fp32_peak,
-                         "unit": "TFLOP/s", "frac": achieved_fp32 / fp32_peak,
-                         "ops_per_eval": OPS_PER_EVAL,
-                         "frac_scan_steps": achieved_scan / fp32_peak if achieved_scan else None,
-                         "scan_steps_note": f"steps {first_scan + 1}..{steps} only (the scanning launches); the "
-                                            "first steps of a forward holdout run are served from sorted "
-                                            "feature values and count their evaluations without scanning them",
-                         "frac_3op": 0.75 * achieved_fp32 / fp32_peak,
-                         "evals_per_s_per_launch": evals_per_launch / avg_score_s,
+            "roofline": {"bound": "hbm", "kernel": scoring_kernel(k, args.kernel), "achieved": achieved_hbm,
+                         "peak": hbm, "unit": "GB/s", "frac": achieved_hbm / hbm, "peak_source": hbm_src,
+                         "note": "one read of D per scoring launch; the scan is bound by instruction issue above it, "
+                                 "and late forward steps read a row's listed near columns instead of the row",
                          "launch_ms": avg_score_s * 1000.0,
-                         "peak_source": f"{sm} SMs x 128 FP32 lanes x {mhz:.0f} MHz (sampled median; "
-                                        "MEASURED_PEAKS.json holds no FP32 figure); work = 4 FP32-pipe ops per "
-                                        "evaluation (sub, mul, add, compare); frac_3op counts the 3 rounded "
-                                        "arithmetic ops only",
-                         "hbm_achieved_gbs": achieved_hbm, "hbm_peak_gbs": hbm, "hbm_peak_source": hbm_src,
-                         "hbm_frac": achieved_hbm / hbm,
-                         "traffic": args.traffic if args.traffic is not None else
-                         (TRAFFIC_PER_PAIR_K64 if 32 < k <= 64 else TRAFFIC_PER_PAIR) * n_val * n_train,
-                         "traffic_source": "command line" if args.traffic is not None else
-                         ("ncu dram__bytes_read.sum + dram__bytes_write.sum of one seeded k_score_tma launch on "
-                          + ("the k = 50, 30000 x 15000 case (1875.4 MB, profiles/k_score_tma_k50_small_ncu.md)"
-                             if 32 < k <= 64 else
-                             "the 16384 x 8192 case (552.4 MB, profiles/k_score_tma_small_ncu.md)")
-                          + ", scaled per (validation row, training row) pair")},
+                         "evals_per_s_per_launch": evals_per_launch / avg_score_s,
+                         "fp32": {"achieved": achieved_fp32, "peak": fp32_peak, "unit": "TFLOP/s",
+                                  "ratio": achieved_fp32 / fp32_peak,
+                                  "ratio_scan_steps": achieved_scan / fp32_peak if achieved_scan else None,
+                                  "ops_per_eval": OPS_PER_EVAL,
+                                  "note": "what an exhaustive scorer would need (sub, mul, add, compare per evaluation) "
+                                          "against the FP32 pipe; above 1 because evaluations that exact bounds rule out "
+                                          f"are not formed; scan steps: {first_scan + 1}..{steps}",
+                                  "peak_source": f"{sm} SMs x 128 FP32 lanes x {mhz:.0f} MHz (sampled median; "
+                                                 "MEASURED_PEAKS.json holds no FP32 figure)"},
+                         "traffic": args.traffic,
+                         "traffic_source": "command line" if args.traffic is not None else None},
             "clocks": clocks,
             "result": {"ordering": [int(x) for x in res["ordering"][:steps]],
                        "errors": [float(x) for x in res["errors"][:steps]]}}

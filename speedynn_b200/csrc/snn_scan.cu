@@ -14,22 +14,28 @@
 // Backward, d = D - s >= D - max s: 0.8 % of bwd-50k's.  A dense scorer is
 // bound by the FP32 pipe on the other 99 %.
 //
-// One warp per (scored row, group of up to 32 candidates), lane = candidate:
+// One warp per (scored row, group of up to 32 candidates), lane = candidate (small
+// forward problems without walks: two warps):
 //   * starting bounds: backward the previous step's k-th distances; forward from
 //     the row's 256 seed columns, for k <= 16 by group minima, above (and where
 //     nobody kept seeds) by putting the seed columns into the lists first;
 //   * the warp streams its row of D, 512 columns at a time, and queues the
 //     columns that any of its candidates may still take (the sign of D - H, H
-//     the group's largest bound, which falls as the lists fill);
+//     the group's largest bound, which falls as the lists fill); forward, those of
+//     two passes at once;
 //   * queued columns are taken in batches, their candidate values gathered
 //     together from `xg`, the candidates packed [group][column][32] (one aligned
 //     128-byte line per column and group, so a gather is one full-width load);
 //     every lane forms its candidate's exact distance and appends it to its
 //     own buffer in shared memory if it may enter the list;
-//   * forward, where the bounds still reach beyond the row's 1,024 nearest columns
-//     (under the committed D), these are taken first: they leave nearly exact
-//     bounds, and the second pass over the row finds little open (k = 50, third
-//     step of 50,021 x 24,989: 38 -> 30 ms) or is not needed;
+//   * forward, the commit may have listed the row's near columns, about 1,024, with
+//     their distances (snn_commit.cu).  These are taken first, without gathers of D
+//     (for long lists their nearest quarter before the others, in place of the
+//     seeds), and the row is streamed only for bounds that reach beyond them: late
+//     steps of fwd-64k 3.5 -> 2.2 ms, of k = 50 8.0 -> 5.8;
+//   * forward without such a list, where the bounds reach beyond the row's 1,024
+//     nearest columns (estimated from the seeds), the same in two passes over the
+//     row (k = 50, third step of 50,021 x 24,989: 38 -> 30 ms);
 //   * when a lane's buffer is half full, all lanes empty theirs together into
 //     their lists, heaps of k_max (distance, column) keys in shared memory (four
 //     children per node: k = 50 selection 335 -> 314 ms against two).  The
@@ -45,13 +51,14 @@
 // with the insertion unrolled at every use the kernel waited for instructions
 // 80 % of the time.
 //
-// What bounds it: instruction issue (55 to 60 % of the slots; the rest is each
-// warp's own chain) well above the D stream: fwd-64k 3.3 ms per late step, 1.3 ms
-// of it the read of D.  Scoring of a whole fwd-64k selection 293 -> 66 ms
-// (80 with the bounds in a kernel of their own and the outliers scanned here
-// with lane = column, 128 columns per exposed load), a backward step of 25,003
-// x 12,502 7.0 -> 1.0 ms, a k = 50 step of 50,021 x 24,989 57 -> 12 ms, a
-// k = 150 step of 8,192 x 4,096 x 19 130 -> 4 ms.
+// What bounds it: instruction issue (72 % of the slots at half of fwd-64k, 37,000
+// instructions per warp of 32,768 columns; 64 % backward, 49 % at k = 50, where
+// the heaps leave 13 warps per SM) well above the D stream.  The gathers' latency
+// is covered by the other warps: with them in flight through shared memory
+// (cp.async, 8 to 16 columns ahead) fwd-64k took 110 to 112 ms against 110,
+// backward 210 to 217 against 204.  Scoring of a whole fwd-64k selection 293 -> 50
+// ms, a backward step of 25,003 x 12,502 7.0 -> 1.0 ms, a late k = 50 step of
+// 50,021 x 24,989 57 -> 6 ms, a k = 150 step of 8,192 x 4,096 x 19 130 -> 3.2 ms.
 #include <float.h>
 #include <math.h>
 #include <stdint.h>
@@ -144,7 +151,8 @@ constexpr int kSeedNone = 0, kSeedHeap = -1;
 // (fwd-64k 118.0 ms a selection; batches of 8 with 20 warps 122.7, with the
 // loads of one batch under the work of the last one at 16 warps 139.6);
 // problems of at most one such wave of warps, whose time is the chain of
-// gathers of one warp, take batches of 16.
+// gathers of one warp, take batches of 16.  Instances that fill heaps from seeds
+// (k > 16) rarely find shared memory for more than 24 warps.
 constexpr int kBatchMany = 4, kBatchFew = 16, kWarpsMany = 28, kWarpsHeap = 24;
 // ... and, forward from given bounds, two warps for each (row, group), each with
 // every other pass over the row; the first one merges the lists (steps 3 to 8 of

@@ -33,3 +33,16 @@ def test_listed_columns_equal_every_pair(n, m, p, k, kind):
             runs.append(sel.run())
     np.testing.assert_array_equal(runs[0]["ordering"], runs[1]["ordering"])
     np.testing.assert_array_equal(runs[0]["errors64"], runs[1]["errors64"])
+
+
+@pytest.mark.parametrize("k", [5, 50])
+def test_listed_columns_across_folds(k):
+    """The same with folds, whose own columns (+inf in D) no list may hold."""
+    s = datagen.generate(16390, 1, 9, n_mag=5, seed=k)
+    runs = []
+    for kernel in (0, 1):
+        with Selector(s.Xtrain, s.ytrain, k_vals=[k], num_features=6, method="forward", k_fold=7) as sel:
+            sel.set_kernel(kernel)
+            runs.append(sel.run())
+    np.testing.assert_array_equal(runs[0]["ordering"], runs[1]["ordering"])
+    np.testing.assert_array_equal(runs[0]["errors64"], runs[1]["errors64"])
