@@ -47,14 +47,14 @@ sys.path.insert(0, ROOT)
 import numpy as np  # noqa: E402
 
 WORKLOAD = "fwd-64k"
-# DRAM bytes per (validation row, training row) pair of one scoring launch, from an
-# ncu capture of a seeded step (dram__bytes_read.sum + dram__bytes_write.sum =
-# 544.2 + 8.3 MB for 8192 x 16384 pairs): the D stream read once plus the small
-# X, bound and label traffic.
-TRAFFIC_PER_PAIR = 552.44e6 / (8192 * 16384)
-# The same for the 64-slot lists (k in (32, 64]), from a seeded step with k = 50
-# on 15,000 x 30,000 pairs: 1845.4 + 29.9 MB.
-TRAFFIC_PER_PAIR_K64 = 1875.35e6 / (15000 * 30000)
+# DRAM bytes per (validation row, training row) pair of one k_scan launch, from ncu
+# captures (dram__bytes_read.sum + dram__bytes_write.sum) of late steps: forward
+# k = 10 on 16,384 x 32,768 pairs 230.2 + 9.0 MB (near columns listed by the commit,
+# not the rows of D), forward k = 50 on 15,000 x 30,000 pairs 570.0 + 8.4 MB,
+# backward k = 5 on 12,500 x 25,000 pairs 1532.6 + 11.7 MB (D read once, and more).
+TRAFFIC_PER_PAIR = 239.21e6 / (16384 * 32768)
+TRAFFIC_PER_PAIR_K64 = 578.35e6 / (15000 * 30000)
+TRAFFIC_PER_PAIR_BACKWARD = 1544.36e6 / (12500 * 25000)
 METRIC = "cand-evals/s (n_val*n_train*candidates per second), greedy forward selection"
 UNIT = "cand-evals/s"
 
@@ -533,8 +533,12 @@ def run_ours(args, world, rank, local):
                                           f"are not formed; scan steps: {first_scan + 1}..{steps}",
                                   "peak_source": f"{sm} SMs x 128 FP32 lanes x {mhz:.0f} MHz (sampled median; "
                                                  "MEASURED_PEAKS.json holds no FP32 figure)"},
-                         "traffic": args.traffic,
-                         "traffic_source": "command line" if args.traffic is not None else None},
+                         "traffic": args.traffic if args.traffic is not None else
+                         (TRAFFIC_PER_PAIR_BACKWARD if backward else TRAFFIC_PER_PAIR_K64 if k > 16 else
+                          TRAFFIC_PER_PAIR) * n_val * n_train,
+                         "traffic_source": "command line" if args.traffic is not None else
+                         "ncu dram__bytes_read.sum + dram__bytes_write.sum of one late k_scan launch on a smaller "
+                         "case (profiles/k_scan_small_ncu.md), scaled per (validation row, training row) pair"},
             "clocks": clocks,
             "result": {"ordering": [int(x) for x in res["ordering"][:steps]],
                        "errors": [float(x) for x in res["errors"][:steps]]}}
