@@ -677,8 +677,11 @@ SNN_API int snn_create(const snn_desc *d, snn_handle **out)
     if (h->plan.cc == 0)
         return bail(fail(SNN_ERR_UNSUPPORTED, "k_max=%d is above the supported maximum of %d", kmax, snn::kScoreMaxK));
     if (!h->desc.backward && !cv) h->stemp_bytes = snn::sort_temp_bytes(h->p, h->ldc);
+    const bool injected = t_fail_alloc != 0;
+    const size_t arena_used = t_arena ? t_arena->used : 0;
     rc = take_buffers(h, h->block, "a problem", [&](Arena &a) { return carve_buffers(h, a); });
-    if (rc == SNN_ERR_NOMEM && h->near_list) {  // the scan does without them
+    if (rc == SNN_ERR_NOMEM && !injected && !d->backward && h->n_cols >= kNearListCols) {  // the scan does without near lists
+        if (t_arena) t_arena->used = arena_used;
         h->near_list = nullptr;
         h->near_info = h->near_next = nullptr;
         h->no_list = true;

@@ -46,3 +46,27 @@ def test_listed_columns_across_folds(k):
             runs.append(sel.run())
     np.testing.assert_array_equal(runs[0]["ordering"], runs[1]["ordering"])
     np.testing.assert_array_equal(runs[0]["errors64"], runs[1]["errors64"])
+
+
+def test_without_memory_for_the_lists():
+    """A problem that fits the device only without its lists runs without them."""
+    import torch
+
+    n, m = 16384, 20000
+    s = datagen.generate(n, m, 9, n_mag=5, seed=3)
+
+    def run():
+        with Selector(s.Xtrain, s.ytrain, s.Xval, s.yval, k_vals=[5], num_features=5, method="forward") as sel:
+            return sel.run()
+
+    want = run()
+    # D 1.31 GB, everything else but the 0.33 GB of lists below 0.1 GB
+    free, _ = torch.cuda.mem_get_info(0)
+    hog = torch.empty(free - 1560 * 10**6, dtype=torch.uint8, device="cuda:0")
+    try:
+        got = run()
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    np.testing.assert_array_equal(got["ordering"], want["ordering"])
+    np.testing.assert_array_equal(got["errors64"], want["errors64"])
