@@ -169,7 +169,9 @@ cudaError_t launch_walk(const Bufs &b, cudaStream_t s);
 // buffers also keep kSeeds near columns per row for the next step's bounds.
 constexpr int kSeedsPerLane = 8;        // seed columns each lane of the commit keeps: the nearest of each eighth of its columns
 constexpr int kSeeds = 32 * kSeedsPerLane;  // seed columns per row
-// list: write b.near_list by the last such commit's b.near_next.
+// list: write b.near_list by the last such commit's b.near_next.  About 1,024
+// columns are aimed at (768: fwd-64k 94.6, k = 50 271.9 ms a selection, 1,400:
+// 95.3 and 272.0, 1,024: 93.9 and 267.8); kNearList leaves room for twice that.
 constexpr int kNearList = 2048;
 cudaError_t launch_commit(const Bufs &b, int backward, int *seeds, float *seed_d, bool list, cudaStream_t s);
 // Known features (a warm start), in their order; start: from the empty matrix of
