@@ -257,14 +257,16 @@ __global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit,
                 ia = __ldg(seeds + j + 2);
                 ib = __ldg(seeds + j + 3);
             }
-            auto least = [&](float4 d, float2 xa, float2 xb) {  // a NaN is left out
+            auto least = [&](float4 d, float2 xa, float2 xb) {  // a NaN is left out, NaN if all are
                 const float2 u = add2(make_float2(d.x, d.y), sq2(sub2(xv2, xa))), v = add2(make_float2(d.z, d.w), sq2(sub2(xv2, xb)));
                 return fminf(fminf(u.x, u.y), fminf(v.x, v.y));
             };
             const float va = least(da, x0, x1), vb = least(db, x2, x3);
 #pragma unroll
             for (int i = 0; i < 8; i += P) {
-                const float v = P == 8 ? fminf(va, vb) : i ? vb : va;
+                // a group of missing values only (all NaN) counts as no column: as NaN it
+                // would shift L and count a smaller entry twice
+                const float v = fminf(P == 8 ? fminf(va, vb) : i ? vb : va, INFINITY);
                 if (__any_sync(kFull, v < L[SEED - 1])) {
 #pragma unroll
                     for (int q = SEED - 1; q > 0; --q) L[q] = fminf(L[q], fmaxf(L[q - 1], v));
