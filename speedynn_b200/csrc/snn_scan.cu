@@ -846,7 +846,10 @@ cudaError_t launch_batch(const Bufs &b, const ScanCall &c)
         if (e != cudaSuccess) return e;
     }
     auto kern = k_scan<BWD, SEED, BATCH>;
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // The limit belongs to the function, not to this call, and an instance serves
+    // many sizes: every call sets the same value, so that threads with other list
+    // lengths do not take it away between here and the launch.
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, c.max_smem);
     if (e != cudaSuccess) return e;
     kern<<<(unsigned)blocks, 32 * warps, smem, c.stream>>>(b, c.n_cand, G, gs, walks, c.own ? 1 : 0, c.gated ? 1 : 0,
                                                    c.probe ? b.n_rows / kProbeRows : 0);

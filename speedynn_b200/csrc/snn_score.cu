@@ -266,7 +266,12 @@ cudaError_t launch_cc(const Bufs &b, int n_cand, const ScorePlan &pl, cudaStream
     const long long blocks = (long long)((b.n_rows + kRows - 1) / kRows) * n_chunks;
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const size_t smem = plan_smem(CC, pl.warps, b.kmax);
-    cudaError_t e = cudaFuncSetAttribute(k_score<CC, BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // The limit belongs to the function, not to this call: every call sets the same
+    // value, so that threads with other list lengths do not take it away before the launch.
+    int dev = 0, max_smem = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_score<CC, BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
     if (e != cudaSuccess) return e;
     k_score<CC, BWD><<<(unsigned)blocks, 32 * pl.warps, smem, s>>>(b, n_cand, pl.warps, n_chunks);
     return cudaGetLastError();
