@@ -542,29 +542,6 @@ static int validate_desc(const snn_desc *d, int *kmax_out)
 // at 32,768), and the lists would be a quarter of D and more.
 constexpr int kNearListCols = 16384;
 
-// Device bytes a handle for this descriptor allocates (buffers of snn_create
-// plus the load staging buffer), for the batch's memory waves.
-static size_t handle_bytes(const snn_desc *d, int kmax)
-{
-    const size_t p = (size_t)d->p, n_cols = (size_t)d->n_train;
-    const bool cv = d->n_val == 0;
-    const size_t n_rows = cv ? n_cols : (size_t)d->n_val;
-    const size_t ldc = (size_t)round_up(d->n_train, snn::kPadCols);
-    const size_t ldr = cv ? ldc : (size_t)round_up((int)n_rows, snn::kPadCols);
-    const size_t M = d->backward ? 0 : 2 * (size_t)snn::kSeeds + p +  // seed columns, distances, bounds, near columns
-                                           (d->n_train >= kNearListCols ? 2 * (size_t)snn::kNearList + 8 : 0);
-    (void)kmax;
-    size_t f = p * ldc + n_rows * ldc + p * (size_t)d->num_k_vals * n_rows + std::max(n_rows, n_cols) * p +
-               n_rows * M + n_cols + n_rows;
-    // sorted feature columns of the first forward step and the sort's buffers
-    if (!d->backward && !cv) f += p * n_rows + 4 * p * ldc + 2 * p + snn::sort_temp_bytes(d->p, (int)ldc) / sizeof(float) + 1;
-    if (d->backward) f += p * n_rows + n_rows;  // kth_prev, dmax
-    const size_t groups = (p + 31) / 32;         // packed candidates of the pruned scan, backward: their extremes
-    f += groups * ldc * 32 + (d->backward ? 2 * groups * ldc + 4 * p : 0);
-    if (!cv) f += p * ldr;
-    return sizeof(float) * f + ((size_t)1 << 20);
-}
-
 // Every buffer of a handle, in one order for counting and for carving.
 static int carve_buffers(snn_handle *h, Arena &a)
 {
@@ -629,6 +606,35 @@ static int carve_buffers(snn_handle *h, Arena &a)
     return carve(a, &h->stage, (size_t)std::max(h->n_rows, h->n_cols) * p, "staging");
 }
 
+// The sizes that a handle's buffers depend on.
+static void set_shape(snn_handle *h, const snn_desc *d, int kmax)
+{
+    h->desc = *d;
+    h->desc.k_vals = nullptr;
+    h->p = d->p;
+    h->cv = d->n_val == 0;
+    h->n_cols = d->n_train;
+    h->n_rows = h->cv ? d->n_train : d->n_val;
+    h->npf = h->cv ? d->n_train / d->k_fold : 1;
+    h->kmax = kmax;
+    h->nk = d->num_k_vals;
+    h->ldc = round_up(h->n_cols, snn::kPadCols);
+    h->ldr = h->cv ? h->ldc : round_up(h->n_rows, snn::kPadCols);
+    if (!d->backward && !h->cv) h->stemp_bytes = snn::sort_temp_bytes(h->p, h->ldc);
+}
+
+// Bytes that a batch problem's handle carves from the wave's arena, for the
+// waves' sizes: counted by the carving itself.
+static size_t handle_bytes(const snn_desc *d, int kmax)
+{
+    snn_handle h;
+    set_shape(&h, d, kmax);
+    Arena count;
+    count.cap = ~(size_t)0 / 2;
+    carve_buffers(&h, count);
+    return count.used + 256;  // the arena's last problem may end anywhere
+}
+
 SNN_API int snn_create(const snn_desc *d, snn_handle **out)
 {
     g_err.clear();
@@ -636,7 +642,6 @@ SNN_API int snn_create(const snn_desc *d, snn_handle **out)
     *out = nullptr;
     int kmax = 0;
     if (int rc = validate_desc(d, &kmax)) return rc;
-    const int cv = d->n_val == 0;
     if (int rc = check_device(d->device)) return rc;
 
     snn_handle *h = new snn_handle();
@@ -646,19 +651,9 @@ SNN_API int snn_create(const snn_desc *d, snn_handle **out)
         if (!strncmp(f, "launch:", 7)) h->inject_launch = atoi(f + 7);
     }
     if (const char *f = getenv("SNN_INJECT_STALL")) h->inject_stall = atoi(f);
-    h->desc = *d;
     h->kvals.assign(d->k_vals, d->k_vals + d->num_k_vals);
-    h->desc.k_vals = nullptr;
     h->device = d->device;
-    h->p = d->p;
-    h->cv = cv;
-    h->n_cols = d->n_train;
-    h->n_rows = cv ? d->n_train : d->n_val;
-    h->npf = cv ? d->n_train / d->k_fold : 1;
-    h->kmax = kmax;
-    h->nk = d->num_k_vals;
-    h->ldc = round_up(h->n_cols, snn::kPadCols);
-    h->ldr = cv ? h->ldc : round_up(h->n_rows, snn::kPadCols);
+    set_shape(h, d, kmax);
     if (d->auto_feature)
         h->total_steps = d->p;
     else
@@ -678,7 +673,6 @@ SNN_API int snn_create(const snn_desc *d, snn_handle **out)
     h->plan = snn::plan_score(kmax, d->p, max_smem);
     if (h->plan.cc == 0)
         return bail(fail(SNN_ERR_UNSUPPORTED, "k_max=%d is above the supported maximum of %d", kmax, snn::kScoreMaxK));
-    if (!h->desc.backward && !cv) h->stemp_bytes = snn::sort_temp_bytes(h->p, h->ldc);
     const bool injected = t_fail_alloc != 0;
     const size_t arena_used = t_arena ? t_arena->used : 0;
     rc = take_buffers(h, h->block, "a problem", [&](Arena &a) { return carve_buffers(h, a); });
