@@ -406,8 +406,9 @@ __global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit,
         if (lane != 0) return;
         const float dense = kDenseCost * (float)gs * (K <= 16 ? 1.0f : K <= 32 ? 1.5f : 2.0f) * (float)b.n_cols;
         const int units = (int)fminf(16.0f * cost / dense, 64.0f);
-        const int old = atomicAdd(&b.st->flat, (1 << 20) + units);
-        if ((old >> 20) + 1 == (int)gridDim.x && (old & 0xfffff) + units > 10 * (int)gridDim.x) b.st->full_scan = 1;
+        // of 64 warps per group, so neither half runs over
+        const unsigned long long all = atomicAdd(&b.st->flat, (1ull << 32) + (unsigned)units) + (1ull << 32) + (unsigned)units;
+        if ((unsigned)(all >> 32) == gridDim.x && (unsigned)all > 10ull * gridDim.x) b.st->full_scan = 1;
     };
     auto choose_walks = [&] {
         // The split with the least estimated cost, from 128 sampled columns (64 for
