@@ -217,11 +217,11 @@ __device__ __forceinline__ unsigned zero_one_miss(float t, float p)
 // prediction vector into lossval[(l * n_cand + slot) * nk + m].  A non-RMSE
 // deciding loss (index 0) also replaces rmse32/rmse64, which best k and the
 // winner are chosen from (no other block reads them then).
-__global__ void __launch_bounds__(256) k_losses(Bufs b, int n_cand)
+__global__ void __launch_bounds__(256) k_losses(Bufs b, int n_cand, int l0)
 {
     __shared__ LossShared S;
     if (b.st->done) return;  // nothing was predicted
-    const int slot = blockIdx.x / b.nk, m = blockIdx.x % b.nk, l = blockIdx.y;
+    const int slot = blockIdx.x / b.nk, m = blockIdx.x % b.nk, l = l0 + blockIdx.y;
     const int n = b.n_rows;
     const float *pred = b.pred + ((size_t)slot * b.nk + m) * n;
     const float *y = b.yr;
@@ -279,7 +279,11 @@ cudaError_t launch_mode_predict(const Bufs &b, int n_cand, cudaStream_t s)
 cudaError_t launch_losses(const Bufs &b, int n_cand, cudaStream_t s)
 {
     if (n_cand <= 0) return cudaSuccess;
-    k_losses<<<dim3(n_cand * b.nk, b.nloss), 256, 0, s>>>(b, n_cand);
+    constexpr int kGridY = 65535;  // longer loss lists take several launches
+    for (int l0 = 0; l0 < b.nloss; l0 += kGridY) {
+        const int nl = b.nloss - l0 < kGridY ? b.nloss - l0 : kGridY;
+        k_losses<<<dim3(n_cand * b.nk, nl), 256, 0, s>>>(b, n_cand, l0);
+    }
     return cudaGetLastError();
 }
 
