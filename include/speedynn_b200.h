@@ -161,7 +161,8 @@ SNN_API int snn_get_results(snn_handle *h, int *ordering, int *mask, float *erro
  * candidate's best k and the winner, and snn_get_errors_all returns all of
  * them for each step's winner.  When loss_ids[0] is not RMSE, errors64 of
  * snn_get_results holds that loss's FP32 value.  Default: {RMSE},
- * regression.  Resets a loaded handle to step 0. */
+ * regression, also after a call that fails for want of memory
+ * (SNN_ERR_NOMEM).  Resets a loaded handle to step 0. */
 SNN_API int snn_set_model(snn_handle *h, const int *loss_ids, int n_losses, int model_type);
 
 /* Every loss of every step, in the reference's selected_errors layout

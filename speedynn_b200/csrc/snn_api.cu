@@ -915,11 +915,21 @@ SNN_API int snn_set_model(snn_handle *h, const int *loss_ids, int n_losses, int 
     if (model_type != 0 && model_type != 1) return fail(SNN_ERR_ARG, "model_type %d is not 0 or 1", model_type);
     SNN_CUDA(cudaSetDevice(h->device));
     SNN_CUDA(cudaStreamSynchronize(h->stream));
-    snn::block_release(h->model_block, true);  // an arena's sub-allocations are freed with the arena
-    h->d_loss_ids = nullptr;
-    h->lossval = h->err_all = nullptr;
+    // a handle whose new buffers cannot be had is a plain one: no launch may see a
+    // loss list or a model without its buffers
+    auto plain = [&] {
+        snn::block_release(h->model_block, true);  // an arena's sub-allocations are freed with the arena
+        h->d_loss_ids = nullptr;
+        h->lossval = h->err_all = nullptr;
+        h->loss_ids.assign(1, 0);
+        h->model = 0;
+    };
+    auto give_up = [&](int code) {
+        plain();
+        return code;
+    };
+    plain();
     h->loss_ids.assign(loss_ids, loss_ids + n_losses);
-    h->model = model_type;
     const size_t nl = (size_t)n_losses, p = (size_t)h->p;
     if (h->extra_losses()) {
         if (int rc = take_buffers(h, h->model_block, "losses", [&](Arena &a) {
@@ -927,14 +937,15 @@ SNN_API int snn_set_model(snn_handle *h, const int *loss_ids, int n_losses, int 
                 if (!e) e = carve(a, &h->lossval, nl * p * h->nk, "losses");
                 return e ? e : carve(a, &h->err_all, nl * p, "losses per step");
             }))
-            return rc;
+            return give_up(rc);
         // on the handle's stream (see the k_vals copy in snn_create); the wait lets
         // the caller reuse loss_ids at once
         SNN_CUDA(cudaMemcpyAsync(h->d_loss_ids, h->loss_ids.data(), sizeof(int) * nl, cudaMemcpyHostToDevice, h->stream));
         SNN_CUDA(cudaStreamSynchronize(h->stream));
     }
     if (model_type == 1)
-        if (int rc = take_lists(h)) return rc;
+        if (int rc = take_lists(h)) return give_up(rc);
+    h->model = model_type;
     if (h->loaded) {
         if (int rc = issue_reset(h)) return rc;
         SNN_CUDA(cudaStreamSynchronize(h->stream));
