@@ -103,15 +103,15 @@ struct snn_handle {
     char *stemp = nullptr;
     size_t stemp_bytes = 0;
     unsigned long long *walked = nullptr;  // columns walked by the sorted second step
-    float *xg = nullptr;          // pruned scan: packed candidates [ceil(p / 32)][ldc][32]
+    float *xg = nullptr;          // pruned scan: packed candidates [ceil(p / 32)][ldc][32], in the staging buffer's place
     float2 *ext = nullptr;        // backward: [ceil(p / 32)][ldc] column extremes
     float4 *fstat = nullptr;      // backward: per-feature mean and range
     int bwd_dense = 0;            // backward: 1 the dense scorer is faster on the loaded data, -1 not known (probe each step)
-    int *walk = nullptr, *n_walk = nullptr;  // forward holdout: problems left to k_walk, and how many
+    int *walk = nullptr, *n_walk = nullptr;  // forward holdout: problems left to k_walk (in sord's place), and how many
     bool sorted_start = true;     // SNN_OPT_SORTED_START
     int2 *near_list = nullptr;  // forward, many columns: the commit's near columns per row
     float4 *near_info = nullptr, *near_next = nullptr;
-    bool no_list = false;         // there was no memory for them
+    int lean = 0;                 // what the device had no room for: 1 the near lists, 2 the pruned scan's buffers too
     bool near_ok = false;         // near_next is the last commit's
     bool list_ok = false;         // near_list holds the current D's near columns
     bool seeds_ok = false;        // seeds hold the current D's seed columns
@@ -330,7 +330,7 @@ int first_seeded(const snn_handle *h)
 }
 bool seeds_for_step(const snn_handle *h, int t)
 {
-    return !h->desc.backward && h->seeds && h->kernel != 1 && t >= first_seeded(h);
+    return !h->desc.backward && h->seeds && h->xg && h->kernel != 1 && t >= first_seeded(h);
 }
 
 // How the automatic choice scores step t by the pruned scan (snn_scan.cu): the
@@ -345,7 +345,7 @@ bool seeds_for_step(const snn_handle *h, int t)
 constexpr int kScanAllCols = 4096;
 int scan_seeding(const snn_handle *h, int t, bool seeded)
 {
-    if (h->kernel != 0 || h->count_filter || h->inject_stall >= 0) return -1;
+    if (!h->xg || h->kernel != 0 || h->count_filter || h->inject_stall >= 0) return -1;
     if (h->desc.backward) return h->bwd_dense == 1 ? -1 : h->prev_ok ? snn::kNoSeeds : snn::kOwnSeeds;
     if (seeded) return snn::kGivenSeeds;
     return t == 0 && h->n_cols <= kScanAllCols ? snn::kOwnSeeds : -1;
@@ -548,6 +548,10 @@ static int carve_buffers(snn_handle *h, Arena &a)
     int rc = SNN_OK;
     const int backward = h->desc.backward;
     const size_t p = (size_t)h->p;
+    h->near_list = nullptr;  // optional ones: an earlier try may have set them
+    h->near_info = h->near_next = nullptr;
+    h->ext = nullptr;
+    h->fstat = nullptr;
     if ((rc = carve(a, &h->XT, p * h->ldc, "X_train"))) return rc;
     if ((rc = carve(a, &h->yc, (size_t)h->n_cols, "y_train"))) return rc;
     if (h->cv) {
@@ -580,30 +584,39 @@ static int carve_buffers(snn_handle *h, Arena &a)
         if ((rc = carve(a, &h->seeds, (size_t)h->n_rows * snn::kSeeds, "seed columns"))) return rc;
         if ((rc = carve(a, &h->seed_d, (size_t)h->n_rows * snn::kSeeds, "seed distances"))) return rc;
         if ((rc = carve(a, &h->sbound, p * h->n_rows, "seed bounds"))) return rc;
-        if (h->n_cols >= kNearListCols && !h->no_list) {
+        if (h->n_cols >= kNearListCols && h->lean < 1) {
             if ((rc = carve(a, &h->near_list, (size_t)h->n_rows * snn::kNearList, "near columns"))) return rc;
             if ((rc = carve(a, &h->near_info, (size_t)h->n_rows, "near columns"))) return rc;
             if ((rc = carve(a, &h->near_next, (size_t)h->n_rows, "near columns"))) return rc;
         }
     }
+    // The staging buffer and the sort's value buffer are used at load only, the
+    // packed candidates and the list of walks afterwards.
     const size_t groups = (p + 31) / 32;
-    if ((rc = carve(a, &h->xg, groups * h->ldc * 32, "packed candidates"))) return rc;
-    if (backward && (rc = carve(a, &h->ext, groups * h->ldc, "column extremes"))) return rc;
-    if (backward && (rc = carve(a, &h->fstat, p, "feature ranges"))) return rc;
+    size_t n_stage = (size_t)std::max(h->n_rows, h->n_cols) * p, n_sord = p * h->ldc;
+    const bool scan = h->lean < 2;
+    if (scan) {
+        n_stage = std::max(n_stage, groups * h->ldc * 32);
+        n_sord = std::max(n_sord, p * h->n_rows);
+        if (backward && (rc = carve(a, &h->ext, groups * h->ldc, "column extremes"))) return rc;
+        if (backward && (rc = carve(a, &h->fstat, p, "feature ranges"))) return rc;
+    }
     if (!backward && !h->cv) {
         const size_t pl = p * h->ldc;
         if ((rc = carve(a, &h->sval, pl, "sorted values"))) return rc;
         // the sort's keys at load, then the second step's candidate values in sorted order
         if ((rc = carve(a, &h->skey, pl, "sort keys"))) return rc;
         if ((rc = carve(a, &h->sidx, pl, "sorted indices"))) return rc;
-        if ((rc = carve(a, &h->sord, pl, "sort values"))) return rc;
+        if ((rc = carve(a, &h->sord, n_sord, "sort values"))) return rc;
         if ((rc = carve(a, &h->soff, 2 * p, "sort offsets"))) return rc;
         if ((rc = carve(a, &h->stemp, h->stemp_bytes, "sort workspace"))) return rc;
         if ((rc = carve(a, &h->walked, 1, "walk counter"))) return rc;
-        if ((rc = carve(a, &h->walk, p * h->n_rows, "walks"))) return rc;
         if ((rc = carve(a, &h->n_walk, 1, "walk count"))) return rc;
+        h->walk = h->sord;
     }
-    return carve(a, &h->stage, (size_t)std::max(h->n_rows, h->n_cols) * p, "staging");
+    if ((rc = carve(a, &h->stage, n_stage, "staging"))) return rc;
+    h->xg = scan ? h->stage : nullptr;
+    return SNN_OK;
 }
 
 // The sizes that a handle's buffers depend on.
@@ -675,14 +688,13 @@ SNN_API int snn_create(const snn_desc *d, snn_handle **out)
         return bail(fail(SNN_ERR_UNSUPPORTED, "k_max=%d is above the supported maximum of %d", kmax, snn::kScoreMaxK));
     const bool injected = t_fail_alloc != 0;
     const size_t arena_used = t_arena ? t_arena->used : 0;
-    rc = take_buffers(h, h->block, "a problem", [&](Arena &a) { return carve_buffers(h, a); });
-    if (rc == SNN_ERR_NOMEM && !injected && !d->backward && h->n_cols >= kNearListCols) {  // the scan does without near lists
-        if (t_arena) t_arena->used = arena_used;
-        h->near_list = nullptr;
-        h->near_info = h->near_next = nullptr;
-        h->no_list = true;
-        cudaGetLastError();
+    // Without room for everything, without what only makes it faster: the near
+    // lists, then the pruned scan.
+    for (;; ++h->lean) {
         rc = take_buffers(h, h->block, "a problem", [&](Arena &a) { return carve_buffers(h, a); });
+        if (rc != SNN_ERR_NOMEM || injected || h->lean == 2) break;
+        if (t_arena) t_arena->used = arena_used;
+        cudaGetLastError();
     }
     if (rc) return bail(rc);
     h->stream = h->block.stream;
@@ -745,7 +757,7 @@ static int load_impl(snn_handle *h, const float *X_train, const float *y_train, 
     // distances decides for the runs on this data, before the wait at the end of
     // the load.  A batch does not wait here; its steps probe by themselves.
     h->bwd_dense = 0;
-    if (h->desc.backward && h->kernel == 0 && snn::scan_worth_probing(h->bufs(), h->p)) {
+    if (h->desc.backward && h->xg && h->kernel == 0 && snn::scan_worth_probing(h->bufs(), h->p)) {
         h->bwd_dense = -1;
         if (wait) {
             const Bufs b = h->bufs();
