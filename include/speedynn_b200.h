@@ -253,6 +253,16 @@ SNN_API int snn_get_setup_timing(snn_handle *h, float *ms);
 
 SNN_API int snn_destroy(snn_handle *h);
 
+/* Closed handles' device memory.  Taking memory from the CUDA driver and giving
+ * it back costs more than a small selection, so blocks of up to 256 MB (at most
+ * 16 of them and 256 MB together in the process, on all devices) are kept for
+ * the next handles after their own is destroyed.  The library gives them back
+ * by itself only when one of its own allocations fails; this call gives them
+ * back at once, for allocations outside the library: those of one device, or
+ * of all devices for device < 0.  Handles in use are not affected; any thread
+ * may call it at any time. */
+SNN_API int snn_release_memory(int device);
+
 /* ---------------------------------------------------------------------------
  * 2b. Batches of independent problems
  *

@@ -74,6 +74,7 @@ def lib():
             "snn_get_neighbours": (ctypes.c_int, [vp, _i32p, _i32p, _i32p, _i32p, _f32p]),
             "snn_get_timing": (ctypes.c_int, [vp, _f64p, _i32p, _f64p, _i32p, _f64p, _i32p]),
             "snn_destroy": (ctypes.c_int, [vp]),
+            "snn_release_memory": (ctypes.c_int, [ctypes.c_int]),
             "snn_set_option": (ctypes.c_int, [vp, ctypes.c_int, ctypes.c_int]),
             "snn_get_neighbours_rows": (ctypes.c_int, [vp, _i32p, ctypes.c_int, _i32p, _f32p]),
             "snn_get_predictions": (ctypes.c_int, [vp, _i32p, ctypes.c_int, _i32p, _i32p, _f32p]),

@@ -1193,6 +1193,13 @@ SNN_API int snn_destroy(snn_handle *h)
     return SNN_OK;
 }
 
+SNN_API int snn_release_memory(int device)
+{
+    g_err.clear();
+    snn::blocks_trim(device);
+    return SNN_OK;
+}
+
 }  // extern "C"
 
 // ===========================================================================

@@ -10,7 +10,7 @@
 // Bounds: at most kSpareBlocks blocks and kSpareBytes bytes are kept in the
 // process; larger blocks go straight back to CUDA, the oldest spare makes room
 // for a newer one, and all of a device's spares are given back when an
-// allocation there fails.  A block is released only after its handle's stream
+// allocation there fails or the program asks (snn_release_memory).  A block is released only after its handle's stream
 // has been waited for, so any thread and stream may take it next; the list is
 // guarded by a mutex.  A device reset frees blocks behind our back: a spare is
 // used only while the driver still knows its allocation by the same buffer id
@@ -144,7 +144,7 @@ void blocks_trim(int device)
     {
         std::lock_guard<std::mutex> lk(g_mu);
         for (size_t i = g_spare.size(); i-- > 0;)
-            if (g_spare[i].device == device) {
+            if (device < 0 || g_spare[i].device == device) {
                 drop.push_back(std::move(g_spare[i]));
                 g_spare.erase(g_spare.begin() + i);
             }

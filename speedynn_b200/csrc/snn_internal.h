@@ -28,7 +28,7 @@ struct Block {
 cudaError_t block_acquire(int device, size_t bytes, Block *out);
 // Give a block back: kept as a spare if it is small and nothing uses it any more (idle), else freed.
 void block_release(Block &b, bool idle);
-// Free a device's spare blocks.
+// Free the spare blocks of a device, or of all devices (device < 0).
 void blocks_trim(int device);
 
 // Selection state kept on the device so that a whole greedy step (score ->

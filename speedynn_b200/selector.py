@@ -15,6 +15,12 @@ def _f32(a):
     return np.ascontiguousarray(a, dtype=np.float32)
 
 
+def release_memory(device=-1):
+    """Give closed problems' device memory (at most 256 MB, kept for the next ones) back to
+    CUDA, for another library's allocations; device -1: of all devices."""
+    check(_lib.lib().snn_release_memory(int(device)))
+
+
 class Selector:
     """Greedy kNN wrapper feature selection on one CUDA device.
 

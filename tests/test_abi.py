@@ -167,3 +167,8 @@ def test_batch_model_arguments_are_checked_without_a_gpu():
         assert L.snn_batch_get_errors_all(h, 0, ptr(out, _f32p), out.size) == _lib.SNN_ERR_STATE
     finally:
         L.snn_batch_destroy(h)
+
+
+def test_release_memory_without_handles(L):
+    assert L.snn_release_memory(-1) == _lib.SNN_OK
+    assert L.snn_release_memory(0) == _lib.SNN_OK

@@ -1,10 +1,10 @@
 """Handles on a device that is nearly full: what only makes a problem faster is
-left out before the problem is refused."""
+left out before the problem is refused; and memory that closed handles keep."""
 import numpy as np
 import pytest
 
 from speedynn_b200 import datagen
-from speedynn_b200.selector import Selector
+from speedynn_b200.selector import Selector, release_memory
 
 pytestmark = pytest.mark.gpu
 
@@ -35,3 +35,29 @@ def test_without_memory_for_the_scan():
         torch.cuda.empty_cache()
     for key in ("ordering", "errors", "errors64"):
         np.testing.assert_array_equal(got[key], want[key], err_msg=key)
+
+
+@pytest.mark.parametrize("device", [0, -1])
+def test_closed_handles_memory_is_given_back(device):
+    import torch
+
+    s = datagen.generate(4096, 4096, 9, n_mag=5, seed=5)
+
+    def run():
+        with Selector(s.Xtrain, s.ytrain, s.Xval, s.yval, k_vals=[5], num_features=2, method="forward") as sel:
+            return sel.run()
+
+    run()  # kernels are loaded
+    release_memory(device)
+    free, _ = torch.cuda.mem_get_info(0)
+    want = run()
+    kept = free - torch.cuda.mem_get_info(0)[0]
+    assert 67 * 10**6 < kept <= 256 * 2**20
+    with Selector(s.Xtrain, s.ytrain, k_vals=[5], num_features=2, method="forward") as sel:
+        release_memory(device)  # a handle in use keeps its own
+        in_use = sel.run()
+        release_memory(device)
+        np.testing.assert_array_equal(sel.run()["errors64"], in_use["errors64"])
+    release_memory(device)
+    assert torch.cuda.mem_get_info(0)[0] == free
+    np.testing.assert_array_equal(run()["errors64"], want["errors64"])
