@@ -239,6 +239,12 @@ SNN_API int snn_set_option(snn_handle *h, int option, int value);
 SNN_API int snn_get_filter_counters(snn_handle *h, unsigned long long *row_chunks, unsigned long long *flagged,
                                     unsigned long long *passed);
 
+/* Near columns that forward commits list for the pruned scan (16,384 training
+ * rows and more): *kept is 1 if the handle has memory for them, *usable the
+ * number of scored rows whose list the last commit left fit for use (256 to
+ * 2,048 columns), 0 if it listed none.  Results never depend on it. */
+SNN_API int snn_get_near_lists(snn_handle *h, int *kept, int *usable);
+
 /* CUDA-event milliseconds of each greedy step of the last run/step calls:
  * score_ms[i] and commit_ms[i] for i < n (0 past the steps run).  Returns the
  * number of steps timed. */

@@ -83,6 +83,7 @@ def lib():
             "snn_get_filter_counters": (ctypes.c_int, [vp, ctypes.POINTER(ctypes.c_ulonglong),
                                                        ctypes.POINTER(ctypes.c_ulonglong),
                                                        ctypes.POINTER(ctypes.c_ulonglong)]),
+            "snn_get_near_lists": (ctypes.c_int, [vp, _i32p, _i32p]),
             "snn_get_step_timing": (ctypes.c_int, [vp, _f32p, _f32p, ctypes.c_int]),
             "snn_get_setup_timing": (ctypes.c_int, [vp, _f32p]),
             "snn_batch_create": (ctypes.c_int, [ctypes.POINTER(SnnDesc), ctypes.c_int, ctypes.c_ulonglong,

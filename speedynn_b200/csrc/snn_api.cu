@@ -1153,6 +1153,23 @@ SNN_API int snn_get_filter_counters(snn_handle *h, unsigned long long *row_chunk
     return SNN_OK;
 }
 
+SNN_API int snn_get_near_lists(snn_handle *h, int *kept, int *usable)
+{
+    g_err.clear();
+    if (!h) return fail(SNN_ERR_ARG, "null handle");
+    SNN_CUDA(cudaSetDevice(h->device));
+    int n = 0;
+    if (h->list_ok) {
+        std::vector<float4> info(h->n_rows);
+        SNN_CUDA(cudaMemcpyAsync(info.data(), h->near_info, sizeof(float4) * info.size(), cudaMemcpyDeviceToHost, h->stream));
+        SNN_CUDA(cudaStreamSynchronize(h->stream));
+        for (const float4 &v : info) n += v.x >= (float)snn::kNearLeast && v.x <= (float)snn::kNearList ? 1 : 0;
+    }
+    if (kept) *kept = h->near_list != nullptr;
+    if (usable) *usable = n;
+    return SNN_OK;
+}
+
 SNN_API int snn_get_step_timing(snn_handle *h, float *score_ms, float *commit_ms, int n)
 {
     g_err.clear();

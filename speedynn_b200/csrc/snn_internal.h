@@ -173,6 +173,7 @@ constexpr int kSeeds = 32 * kSeedsPerLane;  // seed columns per row
 // columns are aimed at (768: fwd-64k 94.6, k = 50 271.9 ms a selection, 1,400:
 // 95.3 and 272.0, 1,024: 93.9 and 267.8); kNearList leaves room for twice that.
 constexpr int kNearList = 2048;
+constexpr int kNearLeast = 256;  // a shorter list is not used: too many bounds reach beyond it, and the row is read for them
 cudaError_t launch_commit(const Bufs &b, int backward, int *seeds, float *seed_d, bool list, cudaStream_t s);
 // Known features (a warm start), in their order; start: from the empty matrix of
 // a forward selection (D need not hold anything).

@@ -83,7 +83,6 @@ constexpr float kQueueCost = 14.0f, kWalkStart = 3000.0f, kWalkCost = 8.0f, kPas
 // per candidate (measured: 30,000 x 15,000 x 38 8 ms, the scan 14 with 68 % open).
 constexpr float kReadCost = 0.25f, kTestCost = 4.0f, kDenseCost = 0.28f;
 constexpr int kProbeRows = 64;
-constexpr int kNearLeast = 256;  // of fewer near columns nothing is gained: the row is read for its others
 static_assert(kSeedsPerLane == 8, "the commit and the scan keep eight seeds per lane");
 static_assert(kQueue >= kSeeds && kQueue >= 128 + 16 + 32, "room for a pass's columns");
 

@@ -174,6 +174,13 @@ class Selector:
         check(_lib.lib().snn_get_filter_counters(self._h, ctypes.byref(a), ctypes.byref(b), ctypes.byref(c)))
         return {"row_chunks": a.value, "flagged": b.value, "passed": c.value}
 
+    def near_lists(self):
+        """Near columns that forward commits list for the pruned scan: whether the problem keeps
+        any, and how many scored rows have a usable list since the last commit."""
+        kept, usable = ctypes.c_int(), ctypes.c_int()
+        check(_lib.lib().snn_get_near_lists(self._h, ctypes.byref(kept), ctypes.byref(usable)))
+        return {"kept": bool(kept.value), "usable": usable.value}
+
     def step_timing(self):
         """Per greedy step of the last run: (score_ms, commit_ms) arrays."""
         n = self.p

@@ -20,6 +20,7 @@ def test_without_memory_for_the_scan():
         return Selector(s.Xtrain, s.ytrain, s.Xval, s.yval, k_vals=[10], num_features=3, method="forward")
 
     torch.cuda.synchronize()
+    release_memory()  # what earlier handles left would make room
     free, _ = torch.cuda.mem_get_info(0)
     with make() as sel:
         took = free - torch.cuda.mem_get_info(0)[0]
