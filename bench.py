@@ -48,13 +48,17 @@ import numpy as np  # noqa: E402
 
 WORKLOAD = "fwd-64k"
 # DRAM bytes per (validation row, training row) pair of one k_scan launch, from ncu
-# captures (dram__bytes_read.sum + dram__bytes_write.sum) of late steps: forward
-# k = 10 on 16,384 x 32,768 pairs 230.2 + 9.0 MB (near columns listed by the commit,
-# not the rows of D), forward k = 50 on 15,000 x 30,000 pairs 570.0 + 8.4 MB,
+# captures (dram__bytes_read.sum + dram__bytes_write.sum) half way through a run:
+# forward k = 10 on 16,384 x 32,768 pairs 230.2 + 9.0 MB (near columns listed by the
+# commit, not the rows of D), forward k = 50 on 15,000 x 30,000 pairs 570.0 + 8.4 MB,
 # backward k = 5 on 12,500 x 25,000 pairs 1532.6 + 11.7 MB (D read once, and more).
+# The dense scorers (--kernel) read D once: 1.03 to 1.04 times its bytes.
 TRAFFIC_PER_PAIR = 239.21e6 / (16384 * 32768)
 TRAFFIC_PER_PAIR_K64 = 578.35e6 / (15000 * 30000)
 TRAFFIC_PER_PAIR_BACKWARD = 1544.36e6 / (12500 * 25000)
+TRAFFIC_PER_PAIR_DENSE = 4 * 1.04
+# Issue slots busy in the same captures.
+ISSUE_BUSY, ISSUE_BUSY_K64, ISSUE_BUSY_BACKWARD = 0.66, 0.50, 0.62
 METRIC = "cand-evals/s (n_val*n_train*candidates per second), greedy forward selection"
 UNIT = "cand-evals/s"
 
@@ -101,9 +105,17 @@ def scoring_kernel(kmax, option=0):
 # FP32-pipe operations per evaluation of an exhaustive scorer: sub, mul, add and
 # compare (the reference's scalar loop).  The pruned scan proves from exact bounds
 # that most evaluations cannot enter a list and does not form them, so against
-# this count it runs above the FP32 pipe's peak; what it cannot do without is one
-# read of D per step.
+# this count it runs above the FP32 pipe's peak.
 OPS_PER_EVAL = 4
+
+
+def first_scan_step(kernel, k, n_train, backward):
+    """First greedy step (from 0) that scans: forward holdout steps 1 and, of up to
+    4,096 columns or with a chosen dense kernel, 2 take their lists from sorted values."""
+    if backward:
+        return 0
+    second = k <= 64 if kernel else k <= 32 and n_train <= 4096
+    return 2 if second else 1
 
 
 def fixture_path(name):
@@ -476,7 +488,8 @@ def run_ours(args, world, rank, local):
     e2e_s = allmax((time.perf_counter() - e0) / args.steps, world)
     sel.close()
 
-    # roofline of the scoring kernel: one D read; beside it the FP32 pipe at OPS_PER_EVAL ops per evaluation
+    # roofline of the scoring kernel: the bytes it moves half way through a run; beside
+    # it the FP32 pipe at OPS_PER_EVAL ops per evaluation
     peaks = {}
     try:
         peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
@@ -490,11 +503,13 @@ def run_ours(args, world, rank, local):
     avg_score_s = score_ms / max(1, score_n) / 1000.0
     evals_per_launch = evals / steps
     achieved_fp32 = OPS_PER_EVAL * evals_per_launch / avg_score_s * 1e-12
-    bytes_per_launch = 4.0 * n_val * n_train
-    achieved_hbm = bytes_per_launch / avg_score_s * 1e-9
-    # the same over the steps that scan every column (forward holdout steps 1
-    # and, of up to 4,096 columns, 2 take their lists from sorted feature values)
-    first_scan = 0 if backward else (2 if k <= 32 and n_train <= 4096 else 1)
+    per_pair, issue_busy = ((TRAFFIC_PER_PAIR_DENSE, None) if args.kernel else
+                            (TRAFFIC_PER_PAIR_BACKWARD, ISSUE_BUSY_BACKWARD) if backward else
+                            (TRAFFIC_PER_PAIR_K64, ISSUE_BUSY_K64) if k > 16 else (TRAFFIC_PER_PAIR, ISSUE_BUSY))
+    traffic = args.traffic if args.traffic is not None else per_pair * n_val * n_train
+    mid_ms = float(step_score[steps // 2]) / args.steps
+    achieved_hbm = traffic / mid_ms * 1e-6
+    first_scan = first_scan_step(args.kernel, k, n_train, backward)
     scan_evals = sum(float(n_val) * n_train * (p - t) for t in range(first_scan, steps))
     scan_s = float(step_score[first_scan:].sum()) / args.steps / 1000.0
     achieved_scan = OPS_PER_EVAL * scan_evals / scan_s * 1e-12 if scan_s > 0 else None
@@ -518,11 +533,13 @@ def run_ours(args, world, rank, local):
                        "note": "(row, 64-column chunk) pairs of the dense TMA-fed scorer's full passes in one selection "
                                "(counted in an extra untimed run, which that scorer takes); flagged = re-scored exactly, passing = held a "
                                "list update candidate"},
-            "roofline": {"bound": "hbm", "kernel": scoring_kernel(k, args.kernel), "achieved": achieved_hbm,
+            "roofline": {"bound": "issue", "kernel": scoring_kernel(k, args.kernel), "achieved": achieved_hbm,
                          "peak": hbm, "unit": "GB/s", "frac": achieved_hbm / hbm, "peak_source": hbm_src,
-                         "note": "one read of D per scoring launch; the scan is bound by instruction issue above it, "
-                                 "and late forward steps read a row's listed near columns instead of the row",
-                         "launch_ms": avg_score_s * 1000.0,
+                         "issue_slots_busy": issue_busy,
+                         "note": f"bytes that the scoring launch of greedy step {steps // 2 + 1} moves (traffic) over "
+                                 "that step's scoring time; the scan is bound by instruction issue (share of busy "
+                                 "slots from the same capture), not by these bytes",
+                         "launch_ms": avg_score_s * 1000.0, "mid_step_ms": mid_ms,
                          "evals_per_s_per_launch": evals_per_launch / avg_score_s,
                          "fp32": {"achieved": achieved_fp32, "peak": fp32_peak, "unit": "TFLOP/s",
                                   "ratio": achieved_fp32 / fp32_peak,
@@ -533,12 +550,10 @@ def run_ours(args, world, rank, local):
                                           f"are not formed; scan steps: {first_scan + 1}..{steps}",
                                   "peak_source": f"{sm} SMs x 128 FP32 lanes x {mhz:.0f} MHz (sampled median; "
                                                  "MEASURED_PEAKS.json holds no FP32 figure)"},
-                         "traffic": args.traffic if args.traffic is not None else
-                         (TRAFFIC_PER_PAIR_BACKWARD if backward else TRAFFIC_PER_PAIR_K64 if k > 16 else
-                          TRAFFIC_PER_PAIR) * n_val * n_train,
+                         "traffic": traffic,
                          "traffic_source": "command line" if args.traffic is not None else
-                         "ncu dram__bytes_read.sum + dram__bytes_write.sum of one late k_scan launch on a smaller "
-                         "case (profiles/k_scan_small_ncu.md), scaled per (validation row, training row) pair"},
+                         "ncu dram__bytes_read.sum + dram__bytes_write.sum of one scoring launch half way through a "
+                         "smaller case, scaled per (validation row, training row) pair"},
             "clocks": clocks,
             "result": {"ordering": [int(x) for x in res["ordering"][:steps]],
                        "errors": [float(x) for x in res["errors"][:steps]]}}

@@ -47,3 +47,11 @@ def test_two_gloo_ranks_take_the_slowest_time():
     for _, _, ms, value in got:
         assert ms == pytest.approx(15.0)
         assert value == pytest.approx(2 * 1.0e9 / 0.015)
+
+
+@pytest.mark.parametrize("kernel,k,n_train,backward,want", [
+    (0, 10, 65536, False, 1), (0, 10, 4096, False, 2), (0, 33, 4096, False, 1), (3, 50, 65536, False, 2),
+    (1, 65, 65536, False, 1), (0, 5, 25000, True, 0), (3, 5, 25000, True, 0)])
+def test_first_scanning_step(kernel, k, n_train, backward, want):
+    import bench
+    assert bench.first_scan_step(kernel, k, n_train, backward) == want
