@@ -42,7 +42,7 @@ struct State {
     int best_k_last;  // best k of the last winner
     int num_final;    // features in the model after the last step
     int full_scan;    // 1: the sorted first steps or the pruned scan leave the step to the dense scorer
-    unsigned long long flat;  // the pruned scan's probe in this step: warps << 32, their estimated cost
+    int flat;         // the pruned scan's probe in this step: warps << 20, their estimated cost
 };
 
 // Everything a kernel needs, passed by value.

@@ -83,6 +83,11 @@ constexpr float kQueueCost = 14.0f, kWalkStart = 3000.0f, kWalkCost = 8.0f, kPas
 // per candidate (measured: 30,000 x 15,000 x 38 8 ms, the scan 14 with 68 % open).
 constexpr float kReadCost = 0.25f, kTestCost = 4.0f, kDenseCost = 0.28f;
 constexpr int kProbeRows = 64;
+// The probe's warps and their cost share State::flat, so no more of them than 11
+// bits count: above 1,023 candidates they are spread over fewer rows.  (With 32
+// bits for each, the code of the instances changed: k = 150 0.5 % slower.)
+constexpr int kProbeWarps = 2047;
+static_assert(64 * kProbeWarps < 1 << 20, "their cost, at most 64 each, has 20 bits");
 static_assert(kSeedsPerLane == 8, "the commit and the scan keep eight seeds per lane");
 static_assert(kQueue >= kSeeds && kQueue >= 128 + 16 + 32, "room for a pass's columns");
 
@@ -405,9 +410,8 @@ __global__ void __launch_bounds__(kBatch == kBatchMany ? 32 : 32 * kMaxSplit,
         if (lane != 0) return;
         const float dense = kDenseCost * (float)gs * (K <= 16 ? 1.0f : K <= 32 ? 1.5f : 2.0f) * (float)b.n_cols;
         const int units = (int)fminf(16.0f * cost / dense, 64.0f);
-        // of 64 warps per group, so neither half runs over
-        const unsigned long long all = atomicAdd(&b.st->flat, (1ull << 32) + (unsigned)units) + (1ull << 32) + (unsigned)units;
-        if ((unsigned)(all >> 32) == gridDim.x && (unsigned)all > 10ull * gridDim.x) b.st->full_scan = 1;
+        const int old = atomicAdd(&b.st->flat, (1 << 20) + units);  // of at most kProbeWarps warps
+        if ((old >> 20) + 1 == (int)gridDim.x && (old & 0xfffff) + units > 10 * (int)gridDim.x) b.st->full_scan = 1;
     };
     auto choose_walks = [&] {
         // The split with the least estimated cost, from 128 sampled columns (64 for
@@ -838,7 +842,9 @@ cudaError_t launch_batch(const Bufs &b, const ScanCall &c)
         if (warps > passes) warps = passes;
     }
     const size_t smem = warps * warp_smem(b.kmax, BATCH, 1 + (BWD ? 1 : 0) + (SEED == kSeedHeap || (SEED > 0 && b.near_list) ? 1 : 0));
-    const long long blocks = (long long)(c.probe ? kProbeRows : b.n_rows) * G;
+    const int probe_rows = G > kProbeWarps / kProbeRows ? (G < kProbeWarps ? kProbeWarps / G : 1) : kProbeRows;
+    long long blocks = (long long)(c.probe ? probe_rows : b.n_rows) * G;
+    if (c.probe && blocks > kProbeWarps) blocks = kProbeWarps;  // the first groups speak for the others
     if (smem > (size_t)c.max_smem || blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const int walks = scan_leaves_walks(b, c.n_cand, BWD);
     if (walks && !c.probe) {
@@ -852,7 +858,7 @@ cudaError_t launch_batch(const Bufs &b, const ScanCall &c)
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, c.max_smem);
     if (e != cudaSuccess) return e;
     kern<<<(unsigned)blocks, 32 * warps, smem, c.stream>>>(b, c.n_cand, G, gs, walks, c.own ? 1 : 0, c.gated ? 1 : 0,
-                                                   c.probe ? b.n_rows / kProbeRows : 0);
+                                                   c.probe ? b.n_rows / probe_rows : 0);
     return cudaGetLastError();
 }
 
