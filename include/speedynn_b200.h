@@ -196,9 +196,10 @@ SNN_API int snn_get_timing(snn_handle *h, double *score_ms, int *score_launches,
 
 /* Options:
  *   SNN_OPT_KERNEL scoring kernel: 0 automatic (a pruned scan for steps that
- *                  have starting bounds -- forward steps from seed columns,
- *                  backward steps after the first -- else 3 for k_max <= 64,
- *                  else 1), 1 rows per lane (any k_max <= 256), 3 row tiles
+ *                  have starting bounds or find some -- forward steps with
+ *                  seed columns, first steps of up to 4,096 training rows,
+ *                  backward steps -- unless it does not pay on the data, else
+ *                  3 for k_max <= 64, else 1), 1 rows per lane (any k_max <= 256), 3 row tiles
  *                  fed by a TMA/mbarrier ring (k_max <= 64).  Results are
  *                  identical; this exists for cross-checks and measurement. */
 #define SNN_OPT_KERNEL 2
@@ -254,7 +255,8 @@ SNN_API int snn_get_step_timing(snn_handle *h, float *score_ms, float *commit_ms
  * full distance over all features for backward elimination
  * (compute_distance_matrix_cpu, speedynn/lib/cpu.c:185-215, plus the per-row
  * maxima of the backward filter), the empty matrix for forward selection
- * (empty_distance_matrix_cpu, cpu.c:171-183).  Every run starts with a reset. */
+ * (empty_distance_matrix_cpu, cpu.c:171-183).  Every run starts from such a
+ * reset: the load's or snn_reset's if nothing has run since, else its own. */
 SNN_API int snn_get_setup_timing(snn_handle *h, float *ms);
 
 SNN_API int snn_destroy(snn_handle *h);

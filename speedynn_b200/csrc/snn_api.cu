@@ -294,8 +294,9 @@ int check_device(int device)
     return SNN_OK;
 }
 
-// The TMA-fed scorer (k_max <= 64) is the automatic choice; option 1 forces
-// the rows-per-lane scorer (any k_max <= 256).
+// Which dense scorer takes the steps that the sorted first steps and the pruned
+// scan leave: the TMA-fed one (k_max <= 64), else, and with option 1, the
+// rows-per-lane scorer (any k_max <= 256).
 bool use_tma(const snn_handle *h) { return h->kernel == 3 || (h->kernel == 0 && snn::score_tma_supported(h->kmax)); }
 
 // The first two forward steps of a holdout problem can run from sorted feature

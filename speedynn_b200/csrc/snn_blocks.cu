@@ -1,10 +1,11 @@
 // snn_blocks.cu -- device memory blocks of the handles, and the spare ones.
 //
 // A handle takes all its buffers from one block (plus one for a loss list and
-// one for kept neighbour lists), because every cudaMalloc and cudaFree costs
-// hundreds of microseconds whatever its size (one pair 0.7 ms on an idle B200;
-// 35 pairs, one per buffer, 6 to 40 ms), and a small selection runs for about
-// one millisecond.  Released small blocks are kept for the next handle, with
+// one for kept neighbour lists), because every cudaMalloc and cudaFree costs up
+// to hundreds of microseconds whatever its size, by machine, and a small selection
+// runs for about one millisecond: with a pair per buffer, about 35, whole passes
+// over 100 x 10 rows took 2.3 ms on one B200 and 4.8 on another, where a pair costs
+// 0.7 ms (now 0.34 and 0.36).  Released small blocks are kept for the next handle, with
 // the stream and events of the handle that used them.
 //
 // Bounds: at most kSpareBlocks blocks and kSpareBytes bytes are kept in the

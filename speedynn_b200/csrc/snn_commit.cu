@@ -64,7 +64,9 @@ __device__ __forceinline__ void store_seeds(float (&sv)[kSeedsPerLane], int (&si
 // row's 172nd and 680th smallest distance; their power law goes on to the
 // 1,024th (snn_scan.cu).  From these, what the next commit lists by: that
 // distance, grown by 1.1 times what the last feature added (`last`: the same of
-// the commit before).  The first features change the dimension most: on normal
+// the commit before, 0 on the first one, also after a warm start).  The factors
+// are fitted to normal data; on others fewer lists may be usable (snn_get_near_lists),
+// which costs time and nothing else.  The first features change the dimension most: on normal
 // data the n-th part of the columns reaches about n times as far under two
 // features as under one, and 4.5 times as far under three as under two (the
 // median rows of fwd-64k and fwd-200k 72 and 50 for n of 64 and 49, then 5.1 and

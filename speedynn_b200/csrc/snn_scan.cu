@@ -151,12 +151,13 @@ constexpr int kSeedNone = 0, kSeedHeap = -1;
 
 // kBatch queued columns are gathered together, and a lane buffers up to twice
 // as many keys before they enter its heap.  Large problems take batches of 4 at
-// 64 registers and 28 warps per SM, which hide the gathers for one another
-// (fwd-64k 118.0 ms a selection; batches of 8 with 20 warps 122.7, with the
-// loads of one batch under the work of the last one at 16 warps 139.6);
-// problems of at most one such wave of warps, whose time is the chain of
-// gathers of one warp, take batches of 16.  Instances that fill heaps from seeds
-// (k > 16) rarely find shared memory for more than 24 warps.
+// 72 registers (two instances spill 4 bytes) and 28 warps per SM, which hide the
+// gathers for one another (fwd-64k 118.0 ms a selection; batches of 8 with 20
+// warps 122.7, with the loads of one batch under the work of the last one at 16
+// warps 139.6); few rows (one_wave), whose time is the chain of gathers of one
+// warp, take batches of 16 at up to 128 registers.  Instances that fill heaps
+// from seeds (k > 16) rarely find shared memory for more than 24 warps (80
+// registers).
 constexpr int kBatchMany = 4, kBatchFew = 16, kWarpsMany = 28, kWarpsHeap = 24;
 // ... and, forward from given bounds, two warps for each (row, group), each with
 // every other pass over the row; the first one merges the lists (steps 3 to 8 of
@@ -815,7 +816,13 @@ int sm_count_scan()
     return n;
 }
 
-// At most one wave of warps: a warp's chain of work is the kernel's time.
+// At most one wave of warps at 28 per SM: a warp's chain of work is the kernel's
+// time.  Long lists leave shared memory for fewer warps, four at k = 150, so there
+// these rows are several waves, but the batches of 16 are the better ones all the
+// same: scoring of six steps of 8,192 columns, k = 20, 50, 150, 256, with 500 rows
+// forward 1.0, 1.6, 3.3, 6.0 against 1.7, 2.7, 5.3, 8.5 ms in batches of 4, with
+// 4,096 rows 1.9, 3.9, 15.1, 28.0 against 2.6, 4.8, 18.5, 39.3, backward 2.7, 4.9,
+// 14.3, 25.2 against 5.8, 5.8, 18.2, 38.8.
 bool one_wave(const Bufs &b, int n_cand)
 {
     return (long long)b.n_rows * scan_groups(n_cand) <= (long long)sm_count_scan() * kWarpsMany;

@@ -379,6 +379,8 @@ __device__ __forceinline__ float warp_kth(float (&v)[V], int K, int lane)
     return __shfl_sync(kFull, sel, (K - 1) / V);
 }
 
+// Seed bounds are for seeded steps that go to this scorer: with kernel option 3,
+// the filter counters or an injected stall (the pruned scan forms its own).
 // k_seed_bounds_exact (K <= L <= 16): the bound of each (candidate, scored row)
 // problem is the K-th smallest exact distance d = fl(D + fl((x_r,c - x_i,c)^2))
 // over ALL kSeeds seed columns of the row (see k_seed_bounds for why any K

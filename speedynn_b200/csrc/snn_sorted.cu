@@ -58,7 +58,6 @@ __device__ __forceinline__ float dist1(float a, float b)
     return d < FLT_MAX ? d : INFINITY;  // NaN and values at or above FLT_MAX never enter
 }
 
-// Sorted insertion of column index v into ix[0..n) (ascending).
 // Ascending bitonic sort of one 64-bit key per lane over the warp.
 __device__ __forceinline__ unsigned long long warp_sort64(unsigned long long key, int lane)
 {
@@ -74,6 +73,7 @@ __device__ __forceinline__ unsigned long long warp_sort64(unsigned long long key
     return key;
 }
 
+// Sorted insertion of column index v into ix[0..n) (ascending).
 __device__ __forceinline__ void insert_idx(int *ix, int n, int v)
 {
     int j = n;
@@ -552,7 +552,8 @@ __device__ __forceinline__ bool walk_lists(const Bufs &b, int r, int slot, float
     return true;
 }
 
-// k_second_step_long: the walk of k_second_step for 32 < k <= 64.
+// k_second_step_long: the walk of k_second_step for 32 < k <= 64 (with a chosen
+// dense kernel only; the automatic choice scans such a step).
 __global__ void __launch_bounds__(256, 8) k_second_step_long(Bufs b, const float *sv, const int *si, const float *xs,
                                                           int n_cand, unsigned long long *walked,
                                                           unsigned long long budget)
